@@ -3,11 +3,11 @@
 // compiler command line overrides them; that is how the tuner builds its candidates.
 #pragma once
 #ifndef DSG_PG_MINBLOCKS
-#define DSG_PG_MINBLOCKS 6      // k_pregate blocks per SM (register cap 65536 / (64 x this))
+#define DSG_PG_MINBLOCKS 3      // k_amp256 blocks per SM (register cap 65536 / (128 x this))
 #endif
 #ifndef DSG_FG_MINBLOCKS
-#define DSG_FG_MINBLOCKS 4      // k_fullgate blocks per SM (register cap 65536 / (128 x this))
+#define DSG_FG_MINBLOCKS 2      // k_fullgate blocks per SM (register cap 65536 / (1024 / rows x this))
 #endif
 #ifndef DSG_FG_ROWS
-#define DSG_FG_ROWS 8           // k_fullgate rows staged in shared memory per block step
+#define DSG_FG_ROWS 4           // k_fullgate grid rows per lane
 #endif

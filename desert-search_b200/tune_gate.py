@@ -27,9 +27,9 @@ BUILD = os.path.join(ROOT, "_build")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++20", "-lineinfo", "-fmad=false", "-Xcompiler", "-fPIC", "-I" + os.path.join(HERE, "csrc"), "-I" + os.path.join(ROOT, "include")]
 
-# (pre-gate blocks per SM), (full-gate blocks per SM, full-gate rows per block step); the first is the default
-PREGATE = [6, 5, 7, 8]
-FULLGATE = [(4, 8), (3, 8), (4, 12), (4, 4)]      # rows x 6 KB of static shared memory (48 KB limit)
+# (pre-gate blocks per SM), (full-gate blocks per SM, full-gate rows per lane); the first is the default
+PREGATE = [3, 4, 2]
+FULLGATE = [(2, 4), (1, 4), (1, 2), (2, 8)]       # grid rows per lane: 2, 4 or 8 (16, 8 or 4 warps a block)
 MIN_GAIN = 0.01
 
 
@@ -117,9 +117,9 @@ def header_text(best_pg, best_fg):
     out = ("// Launch shapes of the gate kernels, as chosen by desert-search_b200/tune_gate.py on a B200 (each candidate\n"
            "// built, checked bit for bit against the default build, and timed with dsg_gate_bench).  A -D on the\n"
            "// compiler command line overrides them; that is how the tuner builds its candidates.\n#pragma once\n")
-    for name, val, what in (("DSG_PG_MINBLOCKS", best_pg["pregate_blocks_per_sm"], "k_pregate blocks per SM (register cap 65536 / (64 x this))"),
-                            ("DSG_FG_MINBLOCKS", best_fg["fullgate_blocks_per_sm"], "k_fullgate blocks per SM (register cap 65536 / (128 x this))"),
-                            ("DSG_FG_ROWS", best_fg["fullgate_rows"], "k_fullgate rows staged in shared memory per block step")):
+    for name, val, what in (("DSG_PG_MINBLOCKS", best_pg["pregate_blocks_per_sm"], "k_amp256 blocks per SM (register cap 65536 / (128 x this))"),
+                            ("DSG_FG_MINBLOCKS", best_fg["fullgate_blocks_per_sm"], "k_fullgate blocks per SM (register cap 65536 / (1024 / rows x this))"),
+                            ("DSG_FG_ROWS", best_fg["fullgate_rows"], "k_fullgate grid rows per lane")):
         out += f"#ifndef {name}\n" + f"#define {name} {val}".ljust(32) + f"// {what}\n#endif\n"
     return out
 
