@@ -74,10 +74,8 @@ struct Round {
 };
 __device__ __forceinline__ uint32_t round_of(const Round &q) { return q.round + (q.round_base ? *q.round_base : 0u); }
 
-// Predicate value of request c at quart (x, z): 2 counted, 1 crossed (bridged river), 0 boundary; -1 with `p`
-// filled when a desert point needs desert_state_finish.
-__device__ __forceinline__ int eval_pred(const FloodCtl &c, const SeedNoise &S, const WorldDev &w, int x, int z, PendingState &p) {
-    if (c.pred == DSG_PRED_DESERT) return desert_state_begin(S, w, x, z, p);
+// Hot-zone and proxy predicates of request c at quart (x, z): 2 counted, 0 boundary.
+__device__ __forceinline__ int eval_pred(const FloodCtl &c, const SeedNoise &S, const WorldDev &w, int x, int z) {
     if (c.pred == DSG_PRED_HOT) return hot_state(S, x, z);
     return proxy_prob(S, w, x, z) >= c.pcut ? 2 : 0;
 }
@@ -132,29 +130,97 @@ static __global__ void k_tile_start(const FloodCtl *__restrict__ ctl, const uint
     request_blocks(T, t, 1u << sb, r, n_list, n_cnt, round, active);
 }
 
+// A whole table to shared memory by the EVAL_THREADS threads of a block, every 16-byte load in flight at once.
+template <class T> __device__ __forceinline__ void copy_words(T *dst, const T *__restrict__ src) {
+    static_assert(sizeof(T) % 16 == 0, "copied in 16-byte words");
+    #pragma unroll
+    for (int k = threadIdx.x; k < int(sizeof(T) / 16); k += EVAL_THREADS) reinterpret_cast<uint4 *>(dst)[k] = __ldg(reinterpret_cast<const uint4 *>(src) + k);
+}
+// Bits 0, 4, .. 28 of m as a byte.
+__device__ __forceinline__ uint32_t every_fourth(uint32_t m) {
+    m &= 0x11111111u; m |= m >> 3; m &= 0x03030303u; m |= m >> 6; m &= 0x000f000fu; m |= m >> 12;
+    return m & 0xffu;
+}
 // Evaluate requested sub-blocks: one block of 256 threads per sub-block, a cell per thread (warp = two rows
 // of 16 cells), written as 16-bit pieces of the P and D rows.  Blocks take runs of consecutive sub-blocks
 // from a round counter (up to 16 at a time when the round is large), which balances sub-blocks of very
 // different cost and keeps a block on one request for many items; the request's noise tables stay in
 // shared memory while it does, so every Perlin lookup is a shared-memory access.  Points the surface grid
 // cannot decide (about one in eight near desert edges) are gathered in shared memory and finished by the
-// first threads of the block, so the exact searches run in full warps instead of as one diverged lane per
-// warp.  Each evaluated sub-block marks its tile and queues it for this round's connect.
+// block's threads, one each, spread over its warps.  Each evaluated sub-block marks its tile and queues it for this
+// round's connect.
+// A round of few sub-blocks is bound by the latency of one: 52 octaves one after another and then the exact searches
+// of one thread took about 48,000 and 10,000 to 60,000 cycles.  While four blocks per sub-block fit the grid
+// (blocks-per-SM x SMs, all resident), the desert predicate is therefore evaluated four lanes per cell
+// (desert_state_begin4) and its pending points by eight lanes each (desert_state_finish_group).  Beyond that the grid
+// is full either way, and the work per cell decides, which is less with one lane (no shuffles, no idle lanes).
 static __global__ void __launch_bounds__(EVAL_THREADS, DSG_EVAL_MINB) k_tile_eval(const FloodCtl *__restrict__ ctl, const SeedNoise *__restrict__ noise,
                                                                    WorldDev w, Tiles T, Round q) {
     __shared__ SeedNoise s_noise;
-    __shared__ PendingState s_pend[EVAL_THREADS];
+    // the patch table of the sub-block under evaluation, then its pending points; or what the split form keeps
+    __shared__ union U {
+        PatchCache patch;
+        PendingState pend[EVAL_THREADS];
+        struct { ExactTab exact; PendingState pend[EVAL_THREADS / 4]; } split;
+    } s_u;
     __shared__ int8_t s_res[EVAL_THREADS];
     __shared__ int s_n;
     __shared__ uint32_t s_run;
     const uint32_t items = *q.n_cnt;
     const uint32_t round = round_of(q);
-    const uint32_t run = max(1u, min(uint32_t(DSG_EVAL_RUN), items / (4 * gridDim.x)));
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    bool only = false;                                    // this block evaluates one given sub-block, and no more
+    if (items * 4 <= gridDim.x) {
+        if (blockIdx.x >= items * 4) return;
+        const uint32_t e = q.n_list[blockIdx.x >> 2], t = e >> 4, sb = e & 15, part = blockIdx.x & 3;
+        const uint32_t pos = T.pos[t];
+        const FloodCtl c = ctl[T.owner[t]];
+        if (c.pred == DSG_PRED_DESERT) {
+            copy_words(&s_noise, noise + c.noise);
+            copy_words(&s_u.split.exact, w.exact);
+            if (threadIdx.x == 0) s_n = 0;
+            const int row = int(sb >> 2) * SUB + int(part) * 4 + (warp >> 1), col0 = int(sb & 3) * SUB + (warp & 1) * 8, col = col0 + (lane >> 2);
+            const int i = int(pos & 0xffff) * TILE + col, j = int(pos >> 16) * TILE + row;
+            const int x = c.qx + (i - c.half) * c.step, z = c.qz + (j - c.half) * c.step;
+            const bool on = i < c.n && j < c.n && x >= -kWorld && x <= kWorld && z >= -kWorld && z <= kWorld;
+            __syncthreads();
+            PendingState p;
+            int slot = -1, v = desert_state_begin4(s_noise, w, on ? x : 0, on ? z : 0, on, p);
+            if (v < 0) { slot = atomicAdd(&s_n, 1); s_u.split.pend[slot] = p; }
+            __syncthreads();
+            for (int k0 = 4 * warp; k0 < s_n; k0 += EVAL_THREADS / 8) {
+                const int k = k0 + (lane >> 3);
+                const bool has = k < s_n;
+                const int res = desert_state_finish_group(w, s_u.split.exact, s_u.split.pend[has ? k : k0], has);
+                if (has && (lane & 7) == 0) s_res[k] = int8_t(res);
+            }
+            __syncthreads();
+            if (slot >= 0) v = s_res[slot];
+            const uint32_t pm = __ballot_sync(0xffffffffu, v > 0), dm = __ballot_sync(0xffffffffu, v == 2);      // bits 0, 4, .. 28
+            if (lane == 0) {
+                uint8_t *b = reinterpret_cast<uint8_t *>(T.bits + size_t(t) * TILE_U64) + row * 8 + (col0 >> 3);
+                b[0] = uint8_t(every_fourth(pm)); b[8 * TILE] = uint8_t(every_fourth(dm));
+            }
+            if (threadIdx.x == 0 && part == 0) {
+                atomicOr(&T.emask[t], 1u << sb);
+                if (atomicExch(&T.mark[t], round + 1) != round + 1) q.w_list[atomicAdd(q.w_cnt, 1u)] = t;
+                atomicAdd(q.evaluated, 1ull);
+            }
+            return;
+        }
+        if (part) return;                                 // the other predicates: one block, as in a large round
+        only = true;
+    }
+    const uint32_t run = max(1u, min(uint32_t(DSG_EVAL_RUN), items / (4 * gridDim.x)));
     int staged = -1;                                      // every thread walks the same items: no shared copy needed
-    for (;;) {
+    bool first = true;
+    for (;; first = false) {
+        if (only && !first) break;
         __syncthreads();                                  // the previous item is done with shared memory
-        if (threadIdx.x == 0) s_run = atomicAdd(q.work, run);
+        // the first run is the block's own, so that a round of few sub-blocks spreads over the SMs (blocks are placed on
+        // the SMs in turn; handed out by the counter alone, 112 sub-blocks fell on 56 SMs, three on some); later runs come
+        // from the counter
+        if (threadIdx.x == 0) s_run = only ? blockIdx.x >> 2 : first ? blockIdx.x * run : gridDim.x * run + atomicAdd(q.work, run);
         __syncthreads();
         const uint32_t begin = s_run;
         if (begin >= items) break;
@@ -168,28 +234,31 @@ static __global__ void __launch_bounds__(EVAL_THREADS, DSG_EVAL_MINB) k_tile_eva
             // only the desert predicate batches exact searches; the others need no barrier unless the noise moved
             const bool exact = c.pred == DSG_PRED_DESERT, stage = staged != c.noise;   // block-uniform
             if (stage) {
-                const uint4 *src = reinterpret_cast<const uint4 *>(noise + c.noise);
-                uint4 *dst = reinterpret_cast<uint4 *>(&s_noise);
-                for (int k = threadIdx.x; k < int(sizeof(SeedNoise) / 16); k += blockDim.x) dst[k] = __ldg(src + k);
+                copy_words(&s_noise, noise + c.noise);
                 staged = c.noise;
             }
             if (exact && threadIdx.x == 0) s_n = 0;
-            if (stage || exact) __syncthreads();
-            int v = 0, slot = -1;
-            if (i < c.n && j < c.n) {
-                const int x = c.qx + (i - c.half) * c.step, z = c.qz + (j - c.half) * c.step;
-                if (x >= -kWorld && x <= kWorld && z >= -kWorld && z <= kWorld) {
-                    PendingState p;
-                    v = eval_pred(c, s_noise, w, x, z, p);
-                    if (v < 0) { slot = atomicAdd(&s_n, 1); s_pend[slot] = p; }
-                }
-            }
+            if (stage) __syncthreads();
+            const int x = c.qx + (i - c.half) * c.step, z = c.qz + (j - c.half) * c.step;
+            const bool on = i < c.n && j < c.n && x >= -kWorld && x <= kWorld && z >= -kWorld && z <= kWorld;
+            int v = 0;
             if (exact) {
+                // the patch: the sub-block's cells, and two quarts of warp (more is rare, and such cells look for themselves)
+                const int bi = int(pos & 0xffff) * TILE + int(sb & 3) * SUB, bj = int(pos >> 16) * TILE + int(sb >> 2) * SUB;
+                patch_build(s_noise, s_u.patch, double(c.qx + (bi - c.half) * c.step) - 2, double(c.qz + (bj - c.half) * c.step) - 2,
+                            double((SUB - 1) * c.step + 4), int(threadIdx.x), EVAL_THREADS);
                 __syncthreads();
-                if (int(threadIdx.x) < s_n) s_res[threadIdx.x] = int8_t(desert_state_finish(w, s_pend[threadIdx.x]));
+                PendingState p;
+                if (on) v = desert_state_begin_patch(s_noise, s_u.patch, w, x, z, p);
+                __syncthreads();                          // the pending points take the patch's place
+                int slot = -1;
+                if (v < 0) { slot = atomicAdd(&s_n, 1); s_u.pend[slot] = p; }
+                __syncthreads();
+                // point k on lane k / 8 of warp k % 8: a warp's lanes take turns where their searches differ
+                if (const int k = lane * (EVAL_THREADS / 32) + warp; k < s_n) s_res[k] = int8_t(desert_state_finish(w, s_u.pend[k]));
                 __syncthreads();
                 if (slot >= 0) v = s_res[slot];
-            }
+            } else if (on) v = eval_pred(c, s_noise, w, x, z);
             const uint32_t pm = __ballot_sync(0xffffffffu, v > 0), dm = __ballot_sync(0xffffffffu, v == 2);
             if (lane == 0) {                              // lanes 0-15: row `row`, lanes 16-31: row + 1
                 uint16_t *b = reinterpret_cast<uint16_t *>(T.bits + size_t(t) * TILE_U64);

@@ -91,24 +91,22 @@ __device__ __forceinline__ double channel_low(const SeedNoise &S, int ch, double
     }
     return s * S.factor[ch];
 }
-__device__ __forceinline__ int64_t q10k(float v) { return int64_t(10000.f * v); }
-__device__ __forceinline__ int64_t depth_q(const WorldDev &w, float c, float e, float wv) {
-    const float v[4] = {c, e, -(fabsf(fabsf(wv) - 0.6666667f) - 0.33333334f) * 3.f, wv};
-    const double off = double(spline_eval(w, v) + 0.015f);
+__device__ __forceinline__ int32_t q10k(float v) { return int32_t(10000.f * v); }
+__device__ __forceinline__ float ridge_fold(float wv) { return -(fabsf(fabsf(wv) - 0.6666667f) - 0.33333334f) * 3.f; }
+__device__ __forceinline__ int32_t depth_of(float spline) {
+    const double off = double(spline + 0.015f);
     return q10k(float(1. - (64 * 4) / 128. - 83. / 160. + off));
+}
+__device__ __forceinline__ int32_t depth_q(const WorldDev &w, float c, float e, float wv) {
+    const float v[4] = {c, e, ridge_fold(wv), wv};
+    return depth_of(spline_eval(w, v));
 }
 // Desert flood state at quart (x, 64, z) (surface.hpp:98-124): 2 desert, 1 river bridged to desert, 0 other.
 // In two parts so callers can batch the points the surface grid cannot decide: desert_state_begin returns the
 // state, or -1 with the climate `p` that desert_state_finish completes (exact depth, then the exact search).
-struct PendingState { int64_t q[6]; float c, e, w; int32_t stage; };
-__device__ __forceinline__ int desert_state_begin(const SeedNoise &S, const WorldDev &w, int x, int z, PendingState &p) {
-    const double px = x + 4. * channel(S, CH_S, x, 0, z);
-    const double pz = z + 4. * channel(S, CH_S, z, x, 0);
-    const float t = float(channel(S, CH_T, px, 0, pz));
-    if (q10k(t) < 5500) return 0;
-    const float c = float(channel(S, CH_C, px, 0, pz)), e = float(channel(S, CH_E, px, 0, pz));
-    const float wv = float(channel(S, CH_W, px, 0, pz)), h = float(channel(S, CH_H, px, 0, pz));
-    int64_t q[6] = {q10k(t), q10k(h), q10k(c), q10k(e), -10000, q10k(wv)};
+struct PendingState { int32_t q[6]; float c, e, w; int32_t stage; };
+__device__ __forceinline__ int desert_state_decide(const WorldDev &w, float t, float c, float e, float wv, float h, PendingState &p) {
+    int32_t q[6] = {q10k(t), q10k(h), q10k(c), q10k(e), -10000, q10k(wv)};
     auto pend = [&](int stage) {
         for (int k = 0; k < 6; k++) p.q[k] = q[k];
         p.c = c; p.e = e; p.w = wv; p.stage = stage;
@@ -124,8 +122,171 @@ __device__ __forceinline__ int desert_state_begin(const SeedNoise &S, const Worl
     if (b < 0) return pend(2);                     // second pick (bridged river) needs it
     return b == 2 ? 1 : 0;
 }
+// The octaves of a channel's two sides follow one another in SeedNoise; the channel order is T H C E shift W.
+constexpr int kChanOff[7] = {0, 4, 8, 26, 34, 40, 46};
+constexpr uint64_t octave_sides() {                // bit i: octave i belongs to side B
+    uint64_t m = 0;
+    for (int c = 0; c < 6; c++) for (int i = (kChanOff[c] + kChanOff[c + 1]) / 2; i < kChanOff[c + 1]; i++) m |= uint64_t(1) << i;
+    return m;
+}
+constexpr uint64_t kSideB = octave_sides();
+// ---------------------------------------------------------------- lattice points of a patch, shared by its cells
+// Most climate octaves vary slowly: the 16 x 16 cells of a sub-block lie within two lattice cells along each axis, so
+// the hashes and gradients of the 3 x 3 lattice columns around them serve every cell.  The block works them out once:
+// per octave the lattice cell of the patch's corner (bx, bz) and per lattice column the gradient terms of its two y
+// corners, (gx, gz, gy * dy), dy = fy and fy - 1 (the climate channels are sampled at y = 0).  A cell then needs no
+// hashing: per corner two multiply-adds, fma(gx, x, fma(gz, z, gy * dy)).  One of the three components is zero, so the
+// inner one is exact or the outer adds a zero, and the value is the reference's u + v rounded once, as in grad_d.
+struct __align__(16) LatticePoint { double gx0, gz0, c0, gx1, gz1, c1; };
+constexpr int kPatchOct = 40;                      // T, H, C, E, W: octaves 0..33 and 40..45 of SeedNoise
+struct __align__(16) PatchCache { double bx[kPatchOct], bz[kPatchOct]; LatticePoint pt[kPatchOct][9]; };
+__device__ __forceinline__ int patch_slot(int i) { return i < 34 ? i : i - 6; }
+// The table of the patch [x0, x0 + ext] x [z0, z0 + ext] (quarts, the warped coordinates included) by `nt` threads.  An
+// octave whose patch spans more than about a lattice cell is left out (bx infinite: no cell is found inside).
+__device__ __forceinline__ void patch_build(const SeedNoise &S, PatchCache &C, double x0, double z0, double ext, int t, int nt) {
+    for (int k = t; k < kPatchOct * 9; k += nt) {
+        const int slot = k / 9, j = k % 9, i = slot < 34 ? slot : slot + 6;
+        const NOct &o = S.oct[i];
+        const uint8_t *P = S.perm[i];
+        const double s = (kSideB >> i & 1) ? 337. / 331. : 1.;
+        const double bx = floor(x0 * s * o.freq + o.ox), bz = floor(z0 * s * o.freq + o.oz);
+        const bool use = ext * s * o.freq < 1.25;
+        if (j == 0) { C.bx[slot] = use ? bx : __longlong_as_double(0x7ff0000000000000ll); C.bz[slot] = bz; }
+        if (!use) continue;
+        const int ix = (int(bx) + j % 3) & 255, iz = (int(bz) + j / 3) & 255, a = P[ix] + o.iy;
+        const int h0 = P[P[a & 255] + iz], h1 = P[P[(a + 1) & 255] + iz];
+        C.pt[slot][j] = {grad_d(S.grad, h0, 1., 0., 0.), grad_d(S.grad, h0, 0., 0., 1.), grad_d(S.grad, h0, 0., o.fy, 0.),
+                         grad_d(S.grad, h1, 1., 0., 0.), grad_d(S.grad, h1, 0., 0., 1.), grad_d(S.grad, h1, 0., o.fy - 1, 0.)};
+    }
+}
+// perlin(o, P, G, x, 0, z) of octave slot `k`, from the patch's table where the point lies in it.
+__device__ __forceinline__ double perlin_patch(const NOct &o, const uint8_t *__restrict__ P, const uint2 *__restrict__ G, const PatchCache &C, int k, double x,
+                                               double z) {
+    double fx = (x + o.ox) - C.bx[k], fz = (z + o.oz) - C.bz[k];
+    // both in [0, 2): compared as integers (a negative number's sign bit is the largest)
+    if (uint32_t(__double2hiint(fx)) >= 0x40000000u || uint32_t(__double2hiint(fz)) >= 0x40000000u) return perlin(o, P, G, x, 0, z);
+    const bool cx = __double2hiint(fx) >= 0x3ff00000, cz = __double2hiint(fz) >= 0x3ff00000;
+    fx -= cx ? 1. : 0.; fz -= cz ? 1. : 0.;        // the fractions x - floor(x), z - floor(z): every step is exact
+    const LatticePoint *q = &C.pt[k][(cz ? 3 : 0) + (cx ? 1 : 0)];
+    const double tx = fade_d(fx), tz = fade_d(fz), ty = o.vy, ex = fx - 1;
+    const auto row = [&](const LatticePoint &a, const LatticePoint &b, double dz) {
+        return lerp_d(ty, lerp_d(tx, fma(a.gx0, fx, fma(a.gz0, dz, a.c0)), fma(b.gx0, ex, fma(b.gz0, dz, b.c0))),
+                          lerp_d(tx, fma(a.gx1, fx, fma(a.gz1, dz, a.c1)), fma(b.gx1, ex, fma(b.gz1, dz, b.c1))));
+    };
+    const double lo = row(q[0], q[1], fz);
+    return lerp_d(tz, lo, row(q[3], q[4], fz - 1));
+}
+// channel(S, ch, x, 0, z) for T, H, C, E, W through the patch's table.
+__device__ __forceinline__ double channel_patch(const SeedNoise &S, const PatchCache &C, int ch, double x, double z) {
+    const int off = S.off[ch], cnt = S.cnt[ch];
+    double a0 = 0, a1 = 0;
+    #pragma unroll 1
+    for (int i = off; i < off + cnt; i++) {
+        const NOct &o = S.oct[i];
+        a0 += o.amp * perlin_patch(o, S.perm[i], S.grad, C, patch_slot(i), x * o.freq, z * o.freq);
+    }
+    const double px = x * (337. / 331.), pz = z * (337. / 331.);
+    #pragma unroll 1
+    for (int i = off + cnt; i < off + 2 * cnt; i++) {
+        const NOct &o = S.oct[i];
+        a1 += o.amp * perlin_patch(o, S.perm[i], S.grad, C, patch_slot(i), px * o.freq, pz * o.freq);
+    }
+    return (a0 + a1) * S.factor[ch];
+}
+// desert_state_begin through the patch's table.
+__device__ __forceinline__ int desert_state_begin_patch(const SeedNoise &S, const PatchCache &C, const WorldDev &w, int x, int z, PendingState &p) {
+    const double px = x + 4. * channel(S, CH_S, x, 0, z);
+    const double pz = z + 4. * channel(S, CH_S, z, x, 0);
+    float t = 0, c = 0, e = 0, wv = 0, h = 0;
+    #pragma unroll 1
+    for (int k = 0; k < 5; k++) {                  // one copy of the octave's code for the five channels
+        const int ch = k == 0 ? CH_T : k == 1 ? CH_C : k == 2 ? CH_E : k == 3 ? CH_W : CH_H;
+        const float v = float(channel_patch(S, C, ch, px, pz));
+        if (k == 0) { t = v; if (q10k(t) < 5500) return 0; }
+        else if (k == 1) c = v;
+        else if (k == 2) e = v;
+        else if (k == 3) wv = v;
+        else h = v;
+    }
+    return desert_state_decide(w, t, c, e, wv, h, p);
+}
+__device__ __forceinline__ int desert_state_begin(const SeedNoise &S, const WorldDev &w, int x, int z, PendingState &p) {
+    const double px = x + 4. * channel(S, CH_S, x, 0, z);
+    const double pz = z + 4. * channel(S, CH_S, z, x, 0);
+    const float t = float(channel(S, CH_T, px, 0, pz));
+    if (q10k(t) < 5500) return 0;
+    const float c = float(channel(S, CH_C, px, 0, pz)), e = float(channel(S, CH_E, px, 0, pz));
+    const float wv = float(channel(S, CH_W, px, 0, pz)), h = float(channel(S, CH_H, px, 0, pz));
+    return desert_state_decide(w, t, c, e, wv, h, p);
+}
+// The same by four lanes per point (the whole warp calls; lanes without a point pass any coordinates): the 52 octaves
+// of a point are spread over the lanes four at a time, every lane adds the four terms in the order of the channel sums
+// (per side from +0, then the sides), and lane 0 of the four decides: its result as desert_state_begin's, the others' 0.
+__device__ __forceinline__ double octave_term(const SeedNoise &S, int i, double x, double y, double z) {
+    const double s = (kSideB >> i & 1) ? 337. / 331. : 1.;      // x * 1. is x: side A is not scaled
+    const NOct &o = S.oct[i];
+    return o.amp * perlin(o, S.perm[i], S.grad, x * s * o.freq, y * s * o.freq, z * s * o.freq);
+}
+// Sum of the `n` octaves from off (side A's, then as many of side B), term k held by lane k & 3 of round k / 4.
+struct SideSum {
+    double acc = 0, a = 0;
+    __device__ __forceinline__ bool add(double t, bool last_a, bool last_b) {       // true: the channel's sum is in a
+        acc += t;
+        if (last_a) { a = acc; acc = 0; }
+        if (last_b) { a += acc; acc = 0; }
+        return last_b;
+    }
+};
+__device__ __forceinline__ int desert_state_begin4(const SeedNoise &S, const WorldDev &w, int x, int z, bool on, PendingState &p) {
+    const int lane = threadIdx.x & 31, o = lane & 3, base = lane & 28;
+    double v[2];                                   // the two shift samples: at (x, 0, z) and at (z, x, 0)
+    {
+        SideSum sum;
+        #pragma unroll 1
+        for (int r = 0; r < 3; r++) {
+            const int k = 4 * r + o, second = k >= 6, i = kChanOff[CH_S] + (second ? k - 6 : k);
+            const double t = octave_term(S, i, second ? z : x, second ? x : 0, second ? 0 : z);
+            #pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int n = 4 * r + j;
+                if (sum.add(__shfl_sync(0xffffffffu, t, base + j), n == 2 || n == 8, n == 5 || n == 11)) (n == 5 ? v[0] : v[1]) = sum.a * S.factor[CH_S];
+            }
+        }
+    }
+    const double px = x + 4. * v[0], pz = z + 4. * v[1];
+    float t;
+    {
+        const double u = octave_term(S, kChanOff[CH_T] + o, px, 0, pz);
+        const double a = __shfl_sync(0xffffffffu, u, base), b = __shfl_sync(0xffffffffu, u, base + 1);
+        const double c = __shfl_sync(0xffffffffu, u, base + 2), d = __shfl_sync(0xffffffffu, u, base + 3);
+        t = float(((0. + a + b) + (0. + c + d)) * S.factor[CH_T]);
+    }
+    const bool warm = on && q10k(t) >= 5500;
+    if (!__any_sync(0xffffffffu, warm)) return 0;
+    // C (18 octaves), E (8), W (6), H (4): nine rounds
+    float c = 0, e = 0, wv = 0, h = 0;
+    SideSum sum;
+    constexpr uint64_t endA = 1ull << 8 | 1ull << 21 | 1ull << 28 | 1ull << 33, endB = 1ull << 17 | 1ull << 25 | 1ull << 31 | 1ull << 35;
+    #pragma unroll 1
+    for (int r = 0; r < 9; r++) {
+        const int k = 4 * r + o;
+        const int i = k < 18 ? kChanOff[CH_C] + k : k < 26 ? kChanOff[CH_E] + k - 18 : k < 32 ? kChanOff[CH_W] + k - 26 : kChanOff[CH_H] + k - 32;
+        const double u = octave_term(S, i, px, 0, pz);
+        #pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int n = 4 * r + j;
+            if (sum.add(__shfl_sync(0xffffffffu, u, base + j), endA >> n & 1, endB >> n & 1)) {
+                if (n == 17) c = float(sum.a * S.factor[CH_C]);
+                else if (n == 25) e = float(sum.a * S.factor[CH_E]);
+                else if (n == 31) wv = float(sum.a * S.factor[CH_W]);
+                else h = float(sum.a * S.factor[CH_H]);
+            }
+        }
+    }
+    return warm && o == 0 ? desert_state_decide(w, t, c, e, wv, h, p) : 0;
+}
 __device__ inline int desert_state_finish(const WorldDev &w, const PendingState &p) {
-    int64_t q[6];
+    int32_t q[6];
     for (int k = 0; k < 6; k++) q[k] = p.q[k];
     q[4] = depth_q(w, p.c, p.e, p.w);
     if (p.stage == 2) return classify_exact(w, q) == 2 ? 1 : 0;
@@ -137,6 +298,29 @@ __device__ inline int desert_state_finish(const WorldDev &w, const PendingState 
     b = grid_lookup(w, q);
     if (b < 0) b = classify_exact(w, q);
     return b == 2 ? 1 : 0;
+}
+// desert_state_finish by a group of 8 lanes (the whole warp calls; `on`: the group has a point), T in shared memory.
+__device__ __forceinline__ int desert_state_finish_group(const WorldDev &w, const ExactTab &T, const PendingState &p, bool on) {
+    int32_t q[6];
+    #pragma unroll
+    for (int k = 0; k < 6; k++) q[k] = p.q[k];
+    const GroupSearch first = classify_group_begin(w, T, q, on);
+    q[4] = depth_of(spline_group(T.spline, p.c, p.e, ridge_fold(p.w), p.w));
+    const int b = classify_group_end(w, q, on, first);
+    // first stage: a river near W = 0 crosses to what lies beyond its bank
+    const bool river = on && p.stage != 2 && (b == 7 || b == 11) && q[5] <= 500 && q[5] >= -500;
+    int res = b == 2 ? (p.stage == 2 ? 1 : 2) : 0;
+    if (__any_sync(0xffffffffu, river)) {
+        q[5] = q[5] >= 0 ? 501 : -501;
+        int b2 = river ? grid_lookup(w, q) : 0;
+        const bool again = river && b2 < 0;
+        if (__any_sync(0xffffffffu, again)) {
+            const int b3 = classify_group_end(w, q, again, classify_group_begin(w, T, q, again));
+            if (again) b2 = b3;
+        }
+        if (river) res = b2 == 2 ? 1 : 0;
+    }
+    return res;
 }
 __device__ inline int desert_state(const SeedNoise &S, const WorldDev &w, int x, int z) {
     PendingState p;

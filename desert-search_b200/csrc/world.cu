@@ -4,6 +4,7 @@
 #include "common.cuh"
 #include "world.cuh"
 #include <algorithm>
+#include <functional>
 #include <cstdlib>
 #include <future>
 #include <memory>
@@ -52,6 +53,37 @@ Blob parse_blob() {
         else throw std::runtime_error("worldgen blob: unknown section");
     }
     return b;
+}
+// The inner nodes of the spline graph, in the order first reached from the root (node 0).
+SplineTab spline_table(const std::vector<SplineDev> &spl) {
+    SplineTab t{};
+    std::vector<int> at(spl.size(), -1), order;
+    // every node reachable from k is sound and the inner nodes from k down fill at most `left` levels
+    const std::function<bool(int, int)> fits = [&](int k, int left) {
+        const SplineDev &s = spl[k];
+        if (s.n == 0) return true;
+        if (left == 0 || s.n < 0 || s.n > 12 || s.axis < 0 || s.axis > 3) return false;
+        for (int j = 0; j < s.n; j++)
+            if (s.kid[j] < 0 || size_t(s.kid[j]) >= spl.size() || (j && !(s.knot[j] > s.knot[j - 1])) || !fits(s.kid[j], left - 1)) return false;
+        return true;
+    };
+    if (spl.empty() || spl[0].n == 0 || !fits(0, kSplineLevels)) throw std::runtime_error("worldgen blob: spline graph does not fit its table");
+    at[0] = 0; order.push_back(0);
+    for (size_t i = 0; i < order.size(); i++) {
+        const SplineDev &s = spl[order[i]];
+        t.axis_n[i] = s.axis | s.n << 8;
+        for (int j = 0; j < s.n; j++) {
+            const int k = s.kid[j];
+            t.knot[i][j] = s.knot[j]; t.slope[i][j] = s.slope[j];
+            if (spl[k].n == 0) { t.kid[i][j] = -1; t.leaf[i][j] = spl[k].value; continue; }
+            if (at[k] < 0) {
+                if (order.size() == size_t(kSplineInner)) throw std::runtime_error("worldgen blob: spline graph does not fit its table");
+                at[k] = int(order.size()); order.push_back(k);
+            }
+            t.kid[i][j] = at[k];
+        }
+    }
+    return t;
 }
 // Depth-0 surface grid.  Axes are the climate parameters T, H, C, E, W (slots 0, 1, 2, 3, 5 of a tree node).
 void build_grid(const Blob &b, WorldDev &w, std::vector<int16_t> &cells) {
@@ -476,8 +508,10 @@ void world_upload(int device) {
     // a worker thread while the caller goes on (the gate, tables and scan do not use them); the entry points
     // that classify exactly wait for them in world_dev().
     auto blob = std::make_shared<const Blob>(b);
+    auto exact = std::make_shared<ExactTab>();
+    exact->spline = spline_table(b.spl);
     g_world = w;
-    g_cand_ready = std::async(std::launch::async, [blob, device] {
+    g_cand_ready = std::async(std::launch::async, [blob, exact, device] {
         cudaStream_t st = nullptr;
         try {
             DSG_CU(cudaSetDevice(device));
@@ -489,6 +523,12 @@ void world_upload(int device) {
                 g_world.cdim[a] = c.cdim[a]; g_world.nccut[a] = c.nccut[a];
                 std::copy(c.ccut[a], c.ccut[a] + 48, g_world.ccut[a]);
             }
+            for (int a = 0; a < 5; a++) {
+                std::fill(exact->cut[a], exact->cut[a] + 48, INT32_MAX);
+                std::copy(c.ccut[a], c.ccut[a] + c.nccut[a], exact->cut[a]);
+                exact->dim[a] = c.cdim[a];
+            }
+            g_world.exact = upload(std::vector<ExactTab>{*exact});
             g_world.cand_off = c.cand_off; g_world.cand = c.cand; g_world.cand_n = c.cand_n;
         } catch (const std::exception &ex) {
             if (st) cudaStreamDestroy(st);
