@@ -329,14 +329,16 @@ __device__ inline int desert_state(const SeedNoise &S, const WorldDev &w, int x,
 }
 // Hot-zone predicate: temperature at the unwarped point >= 0.55 (dsearch_desert.cpp:334).
 __device__ __forceinline__ int hot_state(const SeedNoise &S, int x, int z) { return channel(S, CH_T, x, 0, z) >= 0.55 ? 2 : 0; }
-// Low-octave proxy probability (desert_proxy.hpp:24-31).
-__device__ __forceinline__ float proxy_prob(const SeedNoise &S, const WorldDev &w, int x, int z) {
-    if (channel(S, CH_T, x, 0, z) < 0.55) return 0.f;
-    const double c = channel_low(S, CH_C, x, z, 0, 3), e = channel_low(S, CH_E, x, z, 0, 2);
+// Low-octave proxy probability (desert_proxy.hpp:24-31): the bins of continentalness and erosion, where T >= 0.55.
+__device__ __forceinline__ float proxy_bin(const WorldDev &w, double c, double e) {
     int i = int(floor((c + 0.8) / 0.05)), j = int(floor((e + 1.0) / 0.05));
     i = i < 0 ? 0 : (i > 39 ? 39 : i);
     j = j < 0 ? 0 : (j > 39 ? 39 : j);
     return w.prob[i * 40 + j];
+}
+__device__ __forceinline__ float proxy_prob(const SeedNoise &S, const WorldDev &w, int x, int z) {
+    if (channel(S, CH_T, x, 0, z) < 0.55) return 0.f;
+    return proxy_bin(w, channel_low(S, CH_C, x, z, 0, 3), channel_low(S, CH_E, x, z, 0, 2));
 }
 #endif
 

@@ -12,6 +12,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 namespace dsg {
@@ -40,21 +41,166 @@ template <class F> __device__ __forceinline__ void each_chunk(const DZone *__res
     }
 }
 
+// ---- the proxy over tiles of 32 x 32 cells
+// The cells of a zone lie on a regular grid, so per octave a tile's positions, fractions and fades depend on the column
+// or the row alone, and the lattice columns under the tile are few (3 x 3 at frequency 2^-10, 10 x 10 at 2^-7).  The
+// block works those out once per tile: 32 (fraction, fade) pairs per axis and the gradient terms of the lattice columns
+// (LatticePoint, as the flood engine's patches).  A cell then takes about 35 FP64 instructions per octave and no hashing,
+// where it took 69 and 137 others.  The values are the same doubles: the same expressions, evaluated once per column or row.
+// C and E follow only where a cell of the tile is hot.
+// Measured (B200, 160 zones of about 195 x 195 cells): 412 us before, 266 now; one launch is bound by the latency of its
+// FP64 chains (FP64 pipe 50%, issue 50%, shared-memory wavefronts 61%, 4 blocks of 8 warps per SM by registers).  A cell
+// per thread, every corner loaded, was bound by shared memory (78% of its wavefronts; 350 us); rows that test one by one
+// for a new lattice row serialised (316 us); 2 or 3 blocks per SM without spills 314 and 277 us.
+// A zone narrower than 8 cells is evaluated cell by cell: most of a tile would lie outside it.
+constexpr int PT = 32, POCT = 14;                         // tile side; octaves: T (A 0-1, B 0-1), C 0-2 (A, B), E 0-1 (A, B)
+struct ProxyOct { int oct, side, log2f; };                // octave in SeedNoise, side, -log2 of its frequency
+constexpr ProxyOct kPO[POCT] = {{0, 0, 10}, {1, 0, 8}, {2, 1, 10}, {3, 1, 8}, {8, 0, 9}, {9, 0, 8}, {10, 0, 7}, {17, 1, 9}, {18, 1, 8}, {19, 1, 7},
+                                {26, 0, 9}, {27, 0, 8}, {30, 1, 9}, {31, 1, 8}};
+// lattice columns under 31 steps of 32 quarts (x 337/331 on side B): the span in whole cells, one more and the far corner
+constexpr int lattice_width(int log2f) { return int(31 * 32 * 337.0 / 331.0 / double(1 << log2f)) + 3; }
+constexpr int lattice_base(int k) { int n = 0; for (int i = 0; i < k; i++) n += lattice_width(kPO[i].log2f) * lattice_width(kPO[i].log2f); return n; }
+constexpr int PPTS = lattice_base(POCT), PPTS_T = lattice_base(4);
+template <int K> struct TileLattice { static constexpr int oct = kPO[K].oct, side = kPO[K].side, width = lattice_width(kPO[K].log2f), base = lattice_base(K); };
+static_assert(lattice_width(10) == 3 && lattice_width(9) == 4 && lattice_width(8) == 6 && lattice_width(7) == 10 && PPTS == 498, "tile lattice");
+struct TileOct { double ox, oz, freq, s, fy, vy, amp; int32_t iy, width, base, pad; };
+struct __align__(16) ProxyTile {
+    LatticePoint pt[PPTS];
+    double2 line[2][POCT][PT];                            // [x, z]: (fraction, fade) of each column or row
+    TileOct oct[POCT];
+    alignas(16) uint8_t perm[POCT][256];
+    alignas(4) uint8_t at[2][POCT][PT];                   // its lattice column, counted from the tile's first
+    double factor[3];
+};
+static_assert(sizeof(ProxyTile) <= 48 * 1024, "static shared memory");
+// Position of column or row c of the tile whose first lies at x0 (the argument of the octave's floor).
+__device__ __forceinline__ double tile_pos(const TileOct &o, int axis, int x0, int c) { return double(x0 + 32 * c) * o.s * o.freq + (axis ? o.oz : o.ox); }
+// Octaves k0 .. k1 - 1 of the tile at (x0, z0), of mx x mz cells (columns beyond repeat the last).
+__device__ __forceinline__ void tile_build(ProxyTile &T, const uint2 *__restrict__ grad, int k0, int k1, int p0, int p1, int x0, int z0, int mx, int mz) {
+    for (int t = threadIdx.x; t < (k1 - k0) * 2 * PT; t += 256) {
+        const int c = t % PT, axis = t / PT & 1, k = k0 + t / (2 * PT);
+        const TileOct &o = T.oct[k];
+        const int first = axis ? z0 : x0;
+        const double v = tile_pos(o, axis, first, min(c, (axis ? mz : mx) - 1)), b = floor(v), f = v - b;
+        T.line[axis][k][c] = make_double2(f, fade_d(f));
+        T.at[axis][k][c] = uint8_t(int(b - floor(tile_pos(o, axis, first, 0))));
+    }
+    for (int t = p0 + threadIdx.x; t < p1; t += 256) {
+        int k = k0;
+        while (k + 1 < k1 && t >= T.oct[k + 1].base) k++;
+        const TileOct &o = T.oct[k];
+        const int j = t - o.base, ix = (int(floor(tile_pos(o, 0, x0, 0))) + j % o.width) & 255, iz = (int(floor(tile_pos(o, 1, z0, 0))) + j / o.width) & 255;
+        const uint8_t *P = T.perm[k];
+        const int a = P[ix] + o.iy, h0 = P[(P[a & 255] + iz) & 255], h1 = P[(P[(a + 1) & 255] + iz) & 255];
+        T.pt[t] = {grad_d(grad, h0, 1., 0., 0.), grad_d(grad, h0, 0., 0., 1.), grad_d(grad, h0, 0., o.fy, 0.),
+                   grad_d(grad, h1, 1., 0., 0.), grad_d(grad, h1, 0., 0., 1.), grad_d(grad, h1, 0., o.fy - 1, 0.)};
+    }
+}
+// Sums of octaves k0 .. k1 - 1, amp x perlin(x, 0, z) each, at column cx of the four rows r0 .. r0 + 3 (r0 the same for the
+// whole warp).  Where the four rows lie in one row of lattice cells, which at these frequencies is the usual case,
+// its corners are loaded once and their x terms are shared: corner = gz z + (gx x + gy dy), the inner sum per column,
+// the outer per cell.  (Of the three components one is zero, so one of the two sums is exact or adds a zero, and the
+// value is u + v rounded once, whichever of x and z goes first.)
+struct Sum4 { double v[4]; };
+__device__ __noinline__ Sum4 tile_rows(const ProxyTile &T, int k0, int k1, int cx, int r0) {
+    Sum4 s{{0, 0, 0, 0}};
+    #pragma unroll 1
+    for (int k = k0; k < k1; k++) {
+        const TileOct &o = T.oct[k];
+        const int W = o.width;
+        const double2 x = T.line[0][k][cx];
+        const double ty = o.vy, tx = x.y, amp = o.amp, ex = x.x - 1;
+        const LatticePoint *col = &T.pt[o.base + int(T.at[0][k][cx])];
+        const uint32_t lz = *reinterpret_cast<const uint32_t *>(&T.at[1][k][r0]);      // the four rows' lattice rows
+        const double2 *z = &T.line[1][k][r0];
+        double lo[4], hi[4];
+        #pragma unroll
+        for (int h = 0; h < 2; h++) {                     // the lattice row below the cells, then the one above
+            double (&v)[4] = h ? hi : lo;
+            const LatticePoint *a = col + ((lz & 255) + h) * W, *b = a + 1;
+            if ((lz & 255) == lz >> 24) {
+                const double A0 = fma(a->gx0, x.x, a->c0), A1 = fma(b->gx0, ex, b->c0), A2 = fma(a->gx1, x.x, a->c1), A3 = fma(b->gx1, ex, b->c1);
+                const double g0 = a->gz0, g1 = b->gz0, g2 = a->gz1, g3 = b->gz1;
+                #pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const double dz = h ? z[q].x - 1 : z[q].x;
+                    v[q] = lerp_d(ty, lerp_d(tx, fma(g0, dz, A0), fma(g1, dz, A1)), lerp_d(tx, fma(g2, dz, A2), fma(g3, dz, A3)));
+                }
+            } else {
+                #pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const LatticePoint *c = col + ((lz >> (8 * q) & 255) + h) * W, *d = c + 1;
+                    const double dz = h ? z[q].x - 1 : z[q].x;
+                    v[q] = lerp_d(ty, lerp_d(tx, fma(c->gz0, dz, fma(c->gx0, x.x, c->c0)), fma(d->gz0, dz, fma(d->gx0, ex, d->c0))),
+                                      lerp_d(tx, fma(c->gz1, dz, fma(c->gx1, x.x, c->c1)), fma(d->gz1, dz, fma(d->gx1, ex, d->c1))));
+                }
+            }
+        }
+        #pragma unroll
+        for (int q = 0; q < 4; q++) s.v[q] += amp * lerp_d(z[q].y, lo[q], hi[q]);
+    }
+    return s;
+}
 __global__ void __launch_bounds__(256, DSG_PROXY_MINB) k_proxy(const SeedNoise *__restrict__ noise, const DZone *__restrict__ zones, WorldDev w, float cut,
                                                uint8_t *__restrict__ out, ZoneWork wk) {
-    __shared__ SeedNoise S;                               // the zone's seed: every Perlin lookup from shared memory
+    __shared__ ProxyTile T;
     int staged = -1;
     each_chunk(zones, wk, [&](uint32_t, const DZone &z, int64_t c0, int64_t c1) {
+        const SeedNoise &S = noise[z.seed];
+        if (z.nx < 8 || z.nz < 8) {                       // a strip: most of a tile would lie outside
+            for (int64_t c = c0 + threadIdx.x; c < c1; c += blockDim.x)
+                out[z.off + c] = proxy_prob(S, w, z.x0 + 32 * int(c % z.nx), z.z0 + 32 * int(c / z.nx)) >= cut;
+            return;
+        }
         if (z.seed != staged) {                           // block-uniform: every thread walks the same chunks
             __syncthreads();
-            const uint4 *src = reinterpret_cast<const uint4 *>(noise + z.seed);
-            for (int k = threadIdx.x; k < int(sizeof(SeedNoise) / 16); k += blockDim.x) reinterpret_cast<uint4 *>(&S)[k] = __ldg(src + k);
-            __syncthreads();
+            if (threadIdx.x < POCT) {
+                const int k = threadIdx.x;
+                int oi = 0, side = 0, width = 0, base = 0;
+                [&]<int... K>(std::integer_sequence<int, K...>) {
+                    ((K == k ? void((oi = TileLattice<K>::oct, side = TileLattice<K>::side, width = TileLattice<K>::width, base = TileLattice<K>::base)) : void()), ...);
+                }(std::make_integer_sequence<int, POCT>{});
+                const NOct &o = S.oct[oi];
+                T.oct[k] = {o.ox, o.oz, o.freq, side ? 337. / 331. : 1., o.fy, o.vy, o.amp, o.iy, width, base, 0};
+            }
+            if (threadIdx.x < 3) T.factor[threadIdx.x] = S.factor[threadIdx.x == 0 ? CH_T : threadIdx.x == 1 ? CH_C : CH_E];
+            if (threadIdx.x < POCT * 16) {
+                const int k = threadIdx.x >> 4;
+                int oi = 0;
+                [&]<int... K>(std::integer_sequence<int, K...>) { ((K == k ? void(oi = TileLattice<K>::oct) : void()), ...); }(std::make_integer_sequence<int, POCT>{});
+                reinterpret_cast<uint4 *>(T.perm[k])[threadIdx.x & 15] = __ldg(reinterpret_cast<const uint4 *>(S.perm[oi]) + (threadIdx.x & 15));
+            }
             staged = z.seed;
         }
-        for (int64_t c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-            const int ci = int(c % z.nx), cj = int(c / z.nx);
-            out[z.off + c] = proxy_prob(S, w, z.x0 + 32 * ci, z.z0 + 32 * cj) >= cut;
+        // the zone's tiles, dealt to its chunks in turn
+        const int64_t nch = (int64_t(z.nx) * z.nz + CHUNK - 1) / CHUNK;
+        const int tx = (z.nx + PT - 1) / PT, tz = (z.nz + PT - 1) / PT;
+        for (int64_t t = c0 / CHUNK; t < int64_t(tx) * tz; t += nch) {
+            const int i0 = int(t % tx) * PT, j0 = int(t / tx) * PT, mx = min(PT, z.nx - i0), mz = min(PT, z.nz - j0);
+            const int x0 = z.x0 + 32 * i0, z0 = z.z0 + 32 * j0;
+            __syncthreads();                              // the previous tile is done, the octaves are in place
+            tile_build(T, S.grad, 0, 4, 0, PPTS_T, x0, z0, mx, mz);
+            __syncthreads();
+            const int cx = threadIdx.x & 31, r0 = 4 * (threadIdx.x >> 5);       // a warp has four rows
+            const unsigned rows = r0 < mz ? (1u << min(4, mz - r0)) - 1 : 0;
+            unsigned hot = 0;                             // bit q: the cell in row r0 + q
+            {
+                const Sum4 a = tile_rows(T, 0, 2, cx, r0), b = tile_rows(T, 2, 4, cx, r0);
+                #pragma unroll
+                for (int q = 0; q < 4; q++) if (cx < mx && (rows >> q & 1) && !((a.v[q] + b.v[q]) * T.factor[0] < 0.55)) hot |= 1u << q;
+            }
+            if (__syncthreads_or(hot)) {
+                tile_build(T, S.grad, 4, POCT, PPTS_T, PPTS, x0, z0, mx, mz);
+                __syncthreads();
+            }
+            Sum4 c{{0, 0, 0, 0}}, e{{0, 0, 0, 0}};
+            if (__any_sync(0xffffffffu, hot)) { c = tile_rows(T, 4, 10, cx, r0); e = tile_rows(T, 10, POCT, cx, r0); }
+            #pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (cx < mx && (rows >> q & 1)) {
+                    const float prob = (hot >> q & 1) ? proxy_bin(w, c.v[q] * T.factor[1], e.v[q] * T.factor[2]) : 0.f;
+                    out[z.off + int64_t(j0 + r0 + q) * z.nx + i0 + cx] = prob >= cut;
+                }
         }
     });
 }
