@@ -61,8 +61,10 @@ __global__ void k_phase_list(const uint64_t *__restrict__ seeds, uint32_t n, dou
 }
 
 // Temperature octave -10 of both sides of every listed seed (gate.cuh:59-70, k_init).
-__global__ void __launch_bounds__(128) k_octinit(const uint64_t *__restrict__ seeds, const uint32_t *__restrict__ n_in, uint32_t cap,
+constexpr int OCT_THREADS = 64;
+__global__ void __launch_bounds__(OCT_THREADS) k_octinit(const uint64_t *__restrict__ seeds, const uint32_t *__restrict__ n_in, uint32_t cap,
                                                   Oct *__restrict__ oct) {
+    __shared__ uint8_t perm[256][OCT_THREADS];            // a column per thread
     const uint32_t n = min(*n_in, cap);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < 2 * n; i += gridDim.x * blockDim.x) {
         const uint64_t seed = seeds[i >> 1];
@@ -74,12 +76,11 @@ __global__ void __launch_bounds__(128) k_octinit(const uint64_t *__restrict__ se
         if (side) { fa = c.next(); fb = c.next(); }
         Xoro r{fa ^ kSalt10A, fb ^ kSalt10B};
         const double ox = r.uniform() * 256, oy = r.uniform() * 256, oz = r.uniform() * 256;
-        __align__(16) uint8_t perm[256];
-        for (int k = 0; k < 256; k++) perm[k] = uint8_t(k);
-        for (int k = 0; k < 256; k++) { const int j = k + int(r.below(256 - k)); const uint8_t t = perm[k]; perm[k] = perm[j]; perm[j] = t; }
+        uint8_t *p = &perm[0][threadIdx.x];
+        shuffle_column<OCT_THREADS>(r, p);
         Oct &o = oct[i];
-        #pragma unroll
-        for (int k = 0; k < 16; k++) reinterpret_cast<uint4 *>(o.perm)[k] = reinterpret_cast<const uint4 *>(perm)[k];
+        #pragma unroll 2
+        for (int k = 0; k < 16; k++) reinterpret_cast<uint4 *>(o.perm)[k] = column_words<OCT_THREADS>(p, k);
         const double fl = floor(oy);
         o.ox = ox; o.oz = oz; o.fy = oy - fl; o.vy = fade_fused(oy - fl); o.iy = int(fl);
     }
@@ -157,7 +158,7 @@ void enqueue_batch(State &g, cudaStream_t st, uint64_t start, uint64_t nb, const
     DSG_CU(cudaMemsetAsync(g.d_n, 0, 16, st));
     const unsigned pb = unsigned(std::min<uint64_t>((nb + 255) / 256, uint64_t(device_info().sms) * 64));
     k_phase<<<pb, 256, 0, st>>>(start, nb, double(c.maxph), g.d_s1, g.d_n, g.cap1);
-    k_octinit<<<unsigned(device_info().sms) * 16, 128, 0, st>>>(g.d_s1, g.d_n, g.cap1, g.d_oct);
+    k_octinit<<<unsigned(device_info().sms) * 13, OCT_THREADS, 0, st>>>(g.d_s1, g.d_n, g.cap1, g.d_oct);
     k_amp256<AMP_AA><<<g.pg_blocks, PG_THREADS, 0, st>>>(g.d_oct, g.d_s1, g.d_n, g.cap1, c.pthr, g.t256, g.d_s2, g.d_idx2, g.d_n + 1, g.cap2, nullptr);
     k_fullgate<<<g.fg_blocks, FG_THREADS, 0, st>>>(g.d_oct, g.d_s2, g.d_idx2, g.d_n + 1, g.cap2, c.amp, g.t512, g.d_s3, g.d_a3, g.d_n + 2, g.cap3, nullptr);
     DSG_CU(cudaGetLastError());
@@ -227,7 +228,7 @@ extern "C" int dsg_gate_amps(const uint64_t *seeds, uint32_t n, float *pre, floa
         DSG_CU(cudaMemcpy(d_s, seeds, size_t(n) * 8, cudaMemcpyHostToDevice));
         const uint32_t hn[4] = {n, 0, n, 0};
         DSG_CU(cudaMemcpy(d_n, hn, 16, cudaMemcpyHostToDevice));
-        k_octinit<<<(2 * n + 127) / 128, 128>>>(d_s, d_n, n, d_oct);
+        k_octinit<<<(2 * n + OCT_THREADS - 1) / OCT_THREADS, OCT_THREADS>>>(d_s, d_n, n, d_oct);
         k_amp256<AMP_AA><<<g.pg_blocks, PG_THREADS>>>(d_oct, d_s, d_n, n, -1e30, g.t256, d_o, d_i, d_n + 1, n, d_pre);
         k_fullgate<<<g.fg_blocks, FG_THREADS>>>(d_oct, d_s, nullptr, d_n + 2, n, -1e30f, g.t512, d_o, d_a, d_n + 3, n, d_full);
         DSG_CU(cudaGetLastError());
@@ -317,7 +318,7 @@ extern "C" int dsg_subgate_run(uint64_t start, uint64_t count, double maxph, dou
             DSG_CU(cudaMemsetAsync(g.d_n, 0, 16, st));
             const unsigned pb = unsigned(std::min<uint64_t>((nb + 255) / 256, uint64_t(device_info().sms) * 64));
             k_phase<<<pb, 256, 0, st>>>(start + base, nb, maxph, g.d_s1, g.d_n, g.cap1);
-            k_octinit<<<unsigned(device_info().sms) * 16, 128, 0, st>>>(g.d_s1, g.d_n, g.cap1, g.d_oct);
+            k_octinit<<<unsigned(device_info().sms) * 13, OCT_THREADS, 0, st>>>(g.d_s1, g.d_n, g.cap1, g.d_oct);
             k_amp256<AMP_CPU><<<blocks, PG_THREADS, 0, st>>>(g.d_oct, g.d_s1, g.d_n, g.cap1, thr, tp, g.d_s2, nullptr, g.d_n + 1, g.cap2, nullptr);
             DSG_CU(cudaGetLastError());
             DSG_CU(cudaMemcpyAsync(g.h_n, g.d_n, 16, cudaMemcpyDeviceToHost, st));
@@ -363,7 +364,7 @@ extern "C" int dsg_gate_onepar_run(uint64_t start, uint64_t count, const dsg_gat
             DSG_CU(cudaMemsetAsync(g.d_n, 0, 16, st));
             const unsigned pb = unsigned(std::min<uint64_t>((nb + 255) / 256, uint64_t(device_info().sms) * 64));
             k_phase<<<pb, 256, 0, st>>>(start + base, nb, double(cfg->maxph), g.d_s1, g.d_n, g.cap1);
-            k_octinit<<<unsigned(device_info().sms) * 16, 128, 0, st>>>(g.d_s1, g.d_n, g.cap1, g.d_oct);
+            k_octinit<<<unsigned(device_info().sms) * 13, OCT_THREADS, 0, st>>>(g.d_s1, g.d_n, g.cap1, g.d_oct);
             k_amp256<AMP_ONEPAR><<<blocks, PG_THREADS, 0, st>>>(g.d_oct, g.d_s1, g.d_n, g.cap1, thr, g.t256, g.d_s2, g.d_idx2, g.d_n + 1, g.cap2, nullptr);
             k_fullgate<<<g.fg_blocks, FG_THREADS, 0, st>>>(g.d_oct, g.d_s2, g.d_idx2, g.d_n + 1, g.cap2, cfg->amp, g.t512, g.d_s3, g.d_a3, g.d_n + 2,
                                                           g.cap3, nullptr);
@@ -408,7 +409,7 @@ extern "C" int dsg_gate_onepar_amps(const uint64_t *seeds, uint32_t n, float *pr
             DSG_CU(cudaMemcpyAsync(d_s, seeds, size_t(n) * 8, cudaMemcpyHostToDevice, g.st));
             const uint32_t cnt[4] = {n, 0, 0, 0};
             DSG_CU(cudaMemcpyAsync(d_n, cnt, 16, cudaMemcpyHostToDevice, g.st));
-            k_octinit<<<(2 * n + 127) / 128, 128, 0, g.st>>>(d_s, d_n, n, d_oct);
+            k_octinit<<<(2 * n + OCT_THREADS - 1) / OCT_THREADS, OCT_THREADS, 0, g.st>>>(d_s, d_n, n, d_oct);
             k_amp256<AMP_ONEPAR><<<sub_blocks<AMP_ONEPAR>(), PG_THREADS, 0, g.st>>>(d_oct, d_s, d_n, n, -1e30, g.t256, d_o, nullptr, d_n + 1, n, d_e);
             DSG_CU(cudaGetLastError());
             DSG_CU(cudaMemcpyAsync(pre, d_e, size_t(n) * 8, cudaMemcpyDeviceToHost, g.st));
@@ -434,7 +435,7 @@ extern "C" int dsg_subgate_amps(const uint64_t *seeds, uint32_t n, float *est) {
             DSG_CU(cudaMemcpyAsync(d_s, seeds, size_t(n) * 8, cudaMemcpyHostToDevice, g.st));
             const uint32_t cnt[4] = {n, 0, 0, 0};
             DSG_CU(cudaMemcpyAsync(d_n, cnt, 16, cudaMemcpyHostToDevice, g.st));
-            k_octinit<<<(2 * n + 127) / 128, 128, 0, g.st>>>(d_s, d_n, n, d_oct);
+            k_octinit<<<(2 * n + OCT_THREADS - 1) / OCT_THREADS, OCT_THREADS, 0, g.st>>>(d_s, d_n, n, d_oct);
             k_amp256<AMP_CPU><<<sub_blocks<AMP_CPU>(), PG_THREADS, 0, g.st>>>(d_oct, d_s, d_n, n, -1e30, sub_taps(), d_o, nullptr, d_n + 1, n, d_e);
             DSG_CU(cudaGetLastError());
             DSG_CU(cudaMemcpyAsync(est, d_e, size_t(n) * 8, cudaMemcpyDeviceToHost, g.st));
@@ -482,7 +483,7 @@ extern "C" int dsg_gate_bench(uint64_t start, uint64_t per_step, uint32_t steps,
             if (timed) DSG_CU(cudaEventRecord(ev[2 + 5 * k], g.st));
             k_phase<<<pb, 256, 0, g.st>>>(start + uint64_t(it) * per_step, per_step, double(c.maxph), g.d_s1, g.d_n, g.cap1);
             if (timed) DSG_CU(cudaEventRecord(ev[3 + 5 * k], g.st));
-            k_octinit<<<unsigned(device_info().sms) * 16, 128, 0, g.st>>>(g.d_s1, g.d_n, g.cap1, g.d_oct);
+            k_octinit<<<unsigned(device_info().sms) * 13, OCT_THREADS, 0, g.st>>>(g.d_s1, g.d_n, g.cap1, g.d_oct);
             if (timed) DSG_CU(cudaEventRecord(ev[4 + 5 * k], g.st));
             k_amp256<AMP_AA><<<g.pg_blocks, PG_THREADS, 0, g.st>>>(g.d_oct, g.d_s1, g.d_n, g.cap1, c.pthr, g.t256, g.d_s2, g.d_idx2, g.d_n + 1, g.cap2, nullptr);
             if (timed) DSG_CU(cudaEventRecord(ev[5 + 5 * k], g.st));
@@ -516,7 +517,7 @@ void launch_amps_on(const uint64_t *d_seeds, uint32_t n, void *d_oct, uint32_t *
     Taps256 t256; Taps512 t512;
     gate_taps(taps24, t256, t512);
     Oct *oct = static_cast<Oct *>(d_oct);
-    k_octinit<<<(2 * n + 127) / 128, 128, 0, st>>>(d_seeds, d_counters, n, oct);
+    k_octinit<<<(2 * n + OCT_THREADS - 1) / OCT_THREADS, OCT_THREADS, 0, st>>>(d_seeds, d_counters, n, oct);
     k_amp256<AMP_AA><<<pg_blocks, PG_THREADS, 0, st>>>(oct, d_seeds, d_counters, n, -1e30, t256, d_tmp_seeds, d_tmp_idx, d_counters + 1, n, d_pre);
     k_fullgate<<<fg_blocks, FG_THREADS, 0, st>>>(oct, d_seeds, nullptr, d_counters + 2, n, -1e30f, t512, d_tmp_seeds, d_tmp_amp, d_counters + 3, n, d_full);
 }
@@ -658,7 +659,7 @@ void amps_fp64(const uint64_t *d_seeds, uint32_t n, double *d_pre, double *d_ful
     for (uint32_t b = 0; b < n; b += CH) {
         const uint32_t m = std::min(CH, n - b);
         DSG_CU(cudaMemcpyAsync(cnt, &m, 4, cudaMemcpyHostToDevice, st));
-        k_octinit<<<(2 * m + 127) / 128, 128, 0, st>>>(d_seeds + b, cnt, m, oct);
+        k_octinit<<<(2 * m + OCT_THREADS - 1) / OCT_THREADS, OCT_THREADS, 0, st>>>(d_seeds + b, cnt, m, oct);
         k_g64_tables<<<2 * m, 512, 0, st>>>(oct, tpre, tfull);
         DSG_CU(cudaMemsetAsync(best, 0, size_t(2 * m) * 8, st));
         k_g64_cells<G64_PRE><<<dim3(G64_PRE, 2 * m), 256, 0, st>>>(oct, tpre, S);

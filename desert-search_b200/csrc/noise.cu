@@ -23,6 +23,7 @@ __constant__ uint64_t c_salt[11][2] = {
     {0xd50708086cef4d7cULL, 0x6e1651ecc7f43309ULL}};
 __global__ void __launch_bounds__(64) k_seed_noise(const uint64_t *__restrict__ seeds, uint32_t n, SeedNoise *__restrict__ out,
                                                    const uint32_t *__restrict__ n_dev) {
+    __shared__ uint8_t perm[256][64];                    // a column per octave
     if (n_dev) n = min(n, *n_dev);
     // nonzero octave counts per channel (T 2, H 2, C 9, E 4, shift 3, W 3) and their offsets in SeedNoise
     constexpr int kCnt[6] = {2, 2, 9, 4, 3, 3};
@@ -68,17 +69,19 @@ __global__ void __launch_bounds__(64) k_seed_noise(const uint64_t *__restrict__ 
     Xoro rr{ra ^ salt[0], rb ^ salt[1]};
     NOct o;
     o.ox = rr.uniform() * 256; o.oy = rr.uniform() * 256; o.oz = rr.uniform() * 256;
-    __align__(16) uint8_t perm[256];
-    for (int k = 0; k < 256; k++) perm[k] = uint8_t(k);
-    for (int k = 0; k < 256; k++) { const int q = k + int(rr.below(256 - k)); const uint8_t v = perm[k]; perm[k] = perm[q]; perm[q] = v; }
+    uint8_t *p = &perm[0][t];
+    shuffle_column<64>(rr, p);
     const double w0 = double(1 << (c.len - 1)) / ((1 << c.len) - 1);
     o.freq = ldexp(1.0, c.first + i);
     o.amp = ldexp(w0, -i) * c.amp[i];                    // w0 halved i times (exact), times the amplitude
     const double fl = floor(o.oy);
     o.iy = int(fl); o.fy = o.oy - fl; o.vy = fade_d(o.fy); o.pad = 0;
     S.oct[t] = o;
-    #pragma unroll
-    for (int k = 0; k < 32; k++) reinterpret_cast<uint4 *>(S.perm[t])[k] = reinterpret_cast<const uint4 *>(perm)[k & 15];   // stored twice
+    #pragma unroll 2
+    for (int k = 0; k < 16; k++) {                       // stored twice
+        const uint4 v = column_words<64>(p, k);
+        reinterpret_cast<uint4 *>(S.perm[t])[k] = v; reinterpret_cast<uint4 *>(S.perm[t])[k + 16] = v;
+    }
 }
 }  // namespace
 
