@@ -68,11 +68,13 @@ int run_batch(const dsg_flood_req *reqs, uint32_t n, dsg_area *out, size_t pool_
     std::vector<FloodCtl> ctl(n);
     size_t dir_total = 0;
     int64_t dir_max = 0;
+    bool hot = true;                                     // hot-zone floods alone: their own evaluation kernel
     for (uint32_t r = 0; r < n; r++) {
         const dsg_flood_req &q = reqs[r];
         DSG_ARG(q.step >= 1 && q.half >= 0 && q.half <= 32767, "dsg_flood: need step >= 1 and 0 <= half <= 32767");
         DSG_ARG(q.pred == DSG_PRED_DESERT || q.pred == DSG_PRED_HOT || q.pred == DSG_PRED_PROXY, "dsg_flood: unknown predicate");
         DSG_ARG(int64_t(q.half) * q.step < (int64_t(1) << 30), "dsg_flood: window too large");
+        hot &= q.pred == DSG_PRED_HOT;
         auto it = slot.find(q.seed);
         if (it == slot.end()) { it = slot.emplace(q.seed, int32_t(seeds.size())).first; seeds.push_back(q.seed); }
         FloodCtl &c = ctl[r];
@@ -111,7 +113,7 @@ int run_batch(const dsg_flood_req *reqs, uint32_t n, dsg_area *out, size_t pool_
     uint32_t round = 0;
     for (;; K = std::min(2 * K, 64)) {
         for (int k = 0; k < K; k++, round++)
-            launch_round(g.pool, round, g.d_cnt, nullptr, g.d_cnt + 10, g.d_evals, g.d_ctl, g.d_noise, g.d_dir, g.d_stat, ta, g.grid_eval, g.grid_conn, st);
+            launch_round(g.pool, round, g.d_cnt, nullptr, g.d_cnt + 10, g.d_evals, g.d_ctl, g.d_noise, g.d_dir, g.d_stat, ta, g.grid_eval, g.grid_conn, st, nullptr, hot);
         DSG_CU(cudaGetLastError());
         DSG_CU(cudaMemcpyAsync(g.h_cnt, g.d_cnt, 16 * 4, cudaMemcpyDeviceToHost, st));
         DSG_CU(cudaStreamSynchronize(st));

@@ -979,7 +979,7 @@ void capture_phase(Pipeline &p, Slot &S, int k) {
         for (uint32_t it = 0; it < LOOP_LIMIT; it++) {
             for (uint32_t r = 0; r < 6; r++)
                 launch_round(S.pool, r, S.ctr + C_ROUND, nullptr, S.ctr + C_FERR, S.evals, f.ctl, S.noise, f.dir, f.st, ta, p.grid_eval, p.grid_conn,
-                             S.st, S.ctr + C_BASE);
+                             S.st, S.ctr + C_BASE, k < 2);       // the first two phases flood hot zones
             k_loop_ctl<<<1, 1, 0, S.st>>>(S.ctr, 0, false);
             DSG_CU(cudaGetLastError());
             DSG_CU(cudaMemcpyAsync(S.h_ctr, S.ctr, C_N * 4, cudaMemcpyDeviceToHost, S.st));
@@ -1010,7 +1010,7 @@ void capture_phase(Pipeline &p, Slot &S, int k) {
         DSG_CU(cudaStreamBeginCaptureToGraph(S.body_st, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
         for (uint32_t r = 0; r < 6; r++)
             launch_round(S.pool, r, S.ctr + C_ROUND, nullptr, S.ctr + C_FERR, S.evals, f.ctl, S.noise, f.dir, f.st, ta, p.grid_eval, p.grid_conn,
-                         S.body_st, S.ctr + C_BASE);
+                         S.body_st, S.ctr + C_BASE, k < 2);
         k_loop_ctl<<<1, 1, 0, S.body_st>>>(S.ctr, h, true);
         DSG_CU(cudaGetLastError());
         cudaGraph_t body_out = nullptr;

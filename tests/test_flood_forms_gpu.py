@@ -65,3 +65,24 @@ def test_predicates_mixed_in_one_round(dsg):
     for k in (1, 3, len(reqs)):
         assert dsg.flood_batch(reqs[:k]) == want[:k]
     assert dsg.flood_batch(reqs * 30) == want * 30
+
+
+@pytest.mark.parametrize("step,half,conn8", [(256, 40, True), (128, 63, True), (64, 15, False), (1, 50, False), (256, 3, True)])
+def test_hot_floods_alone(dsg, step, half, conn8):
+    """Batches of hot-zone floods alone have a kernel of their own: one flood, a few, many, several seeds a block."""
+    ss = sites(dsg, 12)
+    want = [libs.orc().flood(s, x, z, step, half, conn8, 2) for s, x, z in ss]
+    reqs = [dsg.flood_req(s, x, z, step, half, conn8, 1) for s, x, z in ss]
+    assert [dsg.flood_batch([r])[0] for r in reqs] == want
+    assert dsg.flood_batch(reqs) == want
+    assert dsg.flood_batch(reqs * 200) == want * 200
+    assert any(a[0] > 1 for a in want)
+
+
+def test_hot_floods_at_the_border(dsg):
+    rng = np.random.default_rng(5)
+    reqs, want = [], []
+    for s, _, _ in sites(dsg, 8):
+        for x, z in [(7499900, int(rng.integers(-7e6, 7e6))), (int(rng.integers(-7e6, 7e6)), -7499900)]:
+            reqs.append(dsg.flood_req(s, x, z, 64, 30, True, 1)); want.append(libs.orc().flood(s, x, z, 64, 30, True, 2))
+    assert dsg.flood_batch(reqs) == want and any(a[7] for a in want)
