@@ -54,6 +54,19 @@ template <class T> void grow(T *&p, uint32_t &cap, size_t need) {
     cap = uint32_t(c);
 }
 
+// Tile pool of one call: a quarter of free memory, at most 16 GiB.  A pool that has reached that size stays: asking for the
+// free memory takes 70 us and, where the driver serves other processes too, a millisecond or many.
+constexpr size_t kPoolMost = size_t(16) << 30;
+size_t pool_bytes() {
+    {
+        Engine &g = E();
+        std::lock_guard<std::mutex> l(g.mu);
+        if (g.pool.cap >= kPoolMost / TilePool::kBytesPerTile) return kPoolMost;
+    }
+    size_t free_b = 0, total_b = 0;
+    DSG_CU(cudaMemGetInfo(&free_b, &total_b));
+    return std::min(free_b / 4, kPoolMost);
+}
 // Run a batch of requests to completion.  Returns DSG_OK, or DSG_OVERFLOW if the tile pool ran out (the
 // affected requests must be rerun with more memory).
 int run_batch(const dsg_flood_req *reqs, uint32_t n, dsg_area *out, size_t pool_bytes, uint64_t *cell_off = nullptr,
@@ -177,11 +190,7 @@ extern "C" int dsg_flood_batch(const dsg_flood_req *reqs, uint32_t n, dsg_area *
     return dsg::guarded([&] {
         DSG_ARG(n == 0 || (reqs && out), "dsg_flood_batch: null pointer");
         if (!n) return DSG_OK;
-        size_t free_b = 0, total_b = 0;
-        DSG_CU(cudaMemGetInfo(&free_b, &total_b));
-        // tile pool: a quarter of free memory, at most 16 GiB
-        const size_t pool = std::min<size_t>(free_b / 4, size_t(16) << 30);
-        return dsg::flood::run_batch(reqs, n, out, pool);
+        return dsg::flood::run_batch(reqs, n, out, dsg::flood::pool_bytes());
     });
 }
 extern "C" int dsg_flood(const dsg_flood_req *req, dsg_area *out) { return dsg_flood_batch(req, 1, out); }
@@ -200,9 +209,6 @@ extern "C" int dsg_flood_batch_cells(const dsg_flood_req *reqs, uint32_t n, dsg_
     return dsg::guarded([&] {
         DSG_ARG(n == 0 || (reqs && out && off && (cap == 0 || xz)), "dsg_flood_batch_cells: null pointer");
         if (!n) { if (off) off[0] = 0; return DSG_OK; }
-        size_t free_b = 0, total_b = 0;
-        DSG_CU(cudaMemGetInfo(&free_b, &total_b));
-        const size_t pool = std::min<size_t>(free_b / 4, size_t(16) << 30);
-        return dsg::flood::run_batch(reqs, n, out, pool, off, xz, cap);
+        return dsg::flood::run_batch(reqs, n, out, dsg::flood::pool_bytes(), off, xz, cap);
     });
 }

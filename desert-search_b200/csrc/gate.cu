@@ -254,14 +254,18 @@ extern "C" int dsg_gate_run(uint64_t start, uint64_t count, const dsg_gate_cfg *
         for (uint64_t base = 0; base < count; base += B) {
             const uint64_t nb = std::min(B, count - base);
             enqueue_batch(g, g.st, start + base, nb, *cfg);
+            // the first survivors come with the counts: a short range needs no second round trip
+            const uint32_t few = std::min(g.cap3, 1024u);
             DSG_CU(cudaMemcpyAsync(g.h_n, g.d_n, 16, cudaMemcpyDeviceToHost, g.st));
+            DSG_CU(cudaMemcpyAsync(g.h_s3, g.d_s3, size_t(few) * 8, cudaMemcpyDeviceToHost, g.st));
+            DSG_CU(cudaMemcpyAsync(g.h_a3, g.d_a3, size_t(few) * 4, cudaMemcpyDeviceToHost, g.st));
             DSG_CU(cudaStreamSynchronize(g.st));
             const uint32_t n1 = g.h_n[0], n2 = g.h_n[1], n3 = g.h_n[2];
             overflow |= n1 > g.cap1 || n2 > g.cap2 || n3 > g.cap3;
             const uint32_t k3 = std::min(n3, g.cap3);
-            if (k3) {
-                DSG_CU(cudaMemcpyAsync(g.h_s3, g.d_s3, size_t(k3) * 8, cudaMemcpyDeviceToHost, g.st));
-                DSG_CU(cudaMemcpyAsync(g.h_a3, g.d_a3, size_t(k3) * 4, cudaMemcpyDeviceToHost, g.st));
+            if (k3 > few) {
+                DSG_CU(cudaMemcpyAsync(g.h_s3 + few, g.d_s3 + few, size_t(k3 - few) * 8, cudaMemcpyDeviceToHost, g.st));
+                DSG_CU(cudaMemcpyAsync(g.h_a3 + few, g.d_a3 + few, size_t(k3 - few) * 4, cudaMemcpyDeviceToHost, g.st));
                 DSG_CU(cudaStreamSynchronize(g.st));
             }
             found.clear();

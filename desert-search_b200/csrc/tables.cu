@@ -285,6 +285,10 @@ __global__ void __launch_bounds__(256) k_tabins(const SeedNoise *__restrict__ no
     }
 }
 
+__global__ void k_fill_f32(float *__restrict__ p, float v, uint32_t n) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = v;
+}
+
 // ---------------------------------------------------------------- host engine
 struct State {
     std::mutex mu;
@@ -353,9 +357,7 @@ void launch_tables(State &g, uint32_t S) { launch_tables(TabJob{g.sc, g.d_in, g.
 
 // Tables + blur + max (+ active list and scan if want_scan) for S seeds already in g.d_in; on g.st.
 void enqueue(State &g, uint32_t S, const dsg_scan_params *sp, uint32_t cap, bool want_scan) {
-    const std::vector<float> ninf(size_t(S) * 2, -1e30f);
-    DSG_CU(cudaMemcpyAsync(g.d_mx, ninf.data(), size_t(S) * 8, cudaMemcpyHostToDevice, g.st));
-    DSG_CU(cudaStreamSynchronize(g.st));                 // ninf is a host temporary
+    k_fill_f32<<<(2 * S + 255) / 256, 256, 0, g.st>>>(g.d_mx, -1e30f, 2 * S);
     launch_tables(g, S);
     if (want_scan) {
         DSG_CU(cudaMemsetAsync(g.d_nact, 0, size_t(S) * 4, g.st));
@@ -365,9 +367,6 @@ void enqueue(State &g, uint32_t S, const dsg_scan_params *sp, uint32_t cap, bool
                                                        nullptr);
     }
     DSG_CU(cudaGetLastError());
-}
-__global__ void k_fill_f32(float *__restrict__ p, float v, uint32_t n) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = v;
 }
 }  // namespace tables
 

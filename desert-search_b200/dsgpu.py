@@ -223,7 +223,7 @@ def proxy(seed, zones):
     """Proxy bitmaps (list of (nz, nx) uint8 arrays) of (x0, z0, nx, nz) zones of one seed."""
     zs = (Zone * len(zones))(*[Zone(*z) for z in zones])
     total = sum(z[2] * z[3] for z in zones)
-    bits = np.zeros(max(total, 1), dtype=np.uint8)
+    bits = np.empty(max(total, 1), dtype=np.uint8)
     _ck(lib.dsg_proxy(C.c_uint64(seed & ((1 << 64) - 1)), zs, C.c_uint32(len(zones)), bits.ctypes.data_as(C.c_void_p)), "dsg_proxy")
     out, off = [], 0
     for z in zones:
@@ -237,6 +237,9 @@ class Component(C.Structure):
                 ("inner", C.c_uint32), ("pick", C.c_int32 * 3)]
 
 
+COMPONENT = np.dtype([("zone", "<u4"), ("first", "<i4"), ("cells", "<u4"), ("minx", "<i4"), ("minz", "<i4"), ("inner", "<u4"), ("pick", "<i4", (3,))])
+
+
 def proxy_components(seeds, zone_seed, zones, min_cells=1, cap=1 << 16):
     """Proxy bitmaps of zones of several seeds and their 8-connected components, labelled on the device
     (dsg_proxy_components): (list of component dicts in zone / first-cell order, list of (nz, nx) bitmaps)."""
@@ -244,14 +247,17 @@ def proxy_components(seeds, zone_seed, zones, min_cells=1, cap=1 << 16):
     zsd = np.ascontiguousarray(zone_seed, dtype=np.uint32)
     zs = (Zone * len(zones))(*[Zone(*z) for z in zones])
     total = sum(z[2] * z[3] for z in zones)
-    bits = np.zeros(max(total, 1), dtype=np.uint8)
-    out = (Component * cap)()
+    # written by the library: neither the bitmaps nor the records' room (2.4 MB by default) is cleared first
+    bits = np.empty(max(total, 1), dtype=np.uint8)
+    out = np.empty(cap, dtype=COMPONENT)
     n = C.c_uint32()
     rc = _ck(lib.dsg_proxy_components(ptr(s, u64p), C.c_uint32(len(s)), ptr(zsd, u32p), zs, C.c_uint32(len(zones)), C.c_uint32(min_cells),
-                                      out, C.c_uint32(cap), C.byref(n), bits.ctypes.data_as(C.c_void_p)), "dsg_proxy_components")
+                                      out.ctypes.data_as(C.c_void_p), C.c_uint32(cap), C.byref(n), bits.ctypes.data_as(C.c_void_p)), "dsg_proxy_components")
     assert rc == DSG_OK, "component capacity exceeded"
-    comps = [{"zone": c.zone, "first": c.first, "cells": c.cells, "minx": c.minx, "minz": c.minz, "inner": c.inner,
-              "pick": tuple(c.pick)} for c in out[:n.value]]
+    names = ("zone", "first", "cells", "minx", "minz", "inner")
+    cols = [out[k][:n.value].tolist() for k in names]
+    picks = map(tuple, out["pick"][:n.value].tolist())
+    comps = [dict(zip(names, c), pick=p) for *c, p in zip(*cols, picks)]
     maps, off = [], 0
     for z in zones:
         maps.append(bits[off: off + z[2] * z[3]].reshape(z[3], z[2]))
