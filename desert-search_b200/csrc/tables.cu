@@ -195,20 +195,33 @@ __global__ void __launch_bounds__(TN, Band<R>::BLOCKS) k_tables(const TabIn *__r
     }
 }
 
-// Active side-A T cells (TA >= ta), compacted per seed in row-major order of discovery.
+// Active side-A T cells (TA >= ta), listed per seed.  A warp reads a row in 16-byte words; most rows have none.
 // Seeds blockIdx.y, blockIdx.y + gridDim.y, ... below *n_dev (n_dev null: seed blockIdx.y of gridDim.y).
-__global__ void k_active(const float *__restrict__ tabs, float ta, int32_t *__restrict__ act, uint32_t *__restrict__ nact,
-                         const uint32_t *__restrict__ n_dev) {
+constexpr int ROW_WARPS = 8;
+__global__ void __launch_bounds__(32 * ROW_WARPS) k_active(const float *__restrict__ tabs, float ta, int32_t *__restrict__ act, uint32_t *__restrict__ nact,
+                                                           const uint32_t *__restrict__ n_dev) {
     const uint32_t ns = n_dev ? *n_dev : gridDim.y;
-    const int cell = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const int row = blockIdx.x * ROW_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     for (uint32_t sd = blockIdx.y; sd < ns; sd += gridDim.y) {
-        const bool on = tabs[size_t(sd) * 6 * TN * TN + cell] >= ta;
-        const uint32_t m = __ballot_sync(0xffffffffu, on);
-        if (!m) continue;
-        uint32_t at = 0;
-        if (lane == __ffs(m) - 1) at = atomicAdd(&nact[sd], uint32_t(__popc(m)));
-        at = __shfl_sync(0xffffffffu, at, __ffs(m) - 1);
-        if (on) act[size_t(sd) * TN * TN + at + __popc(m & ((1u << lane) - 1))] = cell;
+        const float4 *p = reinterpret_cast<const float4 *>(tabs + size_t(sd) * 6 * TN * TN + size_t(row) * TN);
+        uint32_t on = 0;                                     // bit 4 k + c: cell 4 (lane + 32 k) + c of the row
+        #pragma unroll
+        for (int k = 0; k < TN / 128; k++) {
+            const float4 v = p[lane + 32 * k];
+            on |= (uint32_t(v.x >= ta) | uint32_t(v.y >= ta) << 1 | uint32_t(v.z >= ta) << 2 | uint32_t(v.w >= ta) << 3) << (4 * k);
+        }
+        if (!__any_sync(0xffffffffu, on != 0)) continue;
+        int at = __popc(on);                                 // inclusive prefix sum of the lanes' counts
+        #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, at, o); if (lane >= o) at += v; }
+        uint32_t base = 0;
+        if (lane == 31) base = atomicAdd(&nact[sd], uint32_t(at));
+        base = __shfl_sync(0xffffffffu, base, 31) + uint32_t(at - __popc(on));
+        int32_t *to = act + size_t(sd) * TN * TN;
+        for (uint32_t m = on; m; m &= m - 1) {
+            const int q = __ffs(m) - 1;
+            to[base++] = row * TN + 4 * (lane + 32 * (q >> 2)) + (q & 3);
+        }
     }
 }
 
@@ -362,7 +375,7 @@ void enqueue(State &g, uint32_t S, const dsg_scan_params *sp, uint32_t cap, bool
     if (want_scan) {
         DSG_CU(cudaMemsetAsync(g.d_nact, 0, size_t(S) * 4, g.st));
         DSG_CU(cudaMemsetAsync(g.d_ncand, 0, size_t(S) * 4, g.st));
-        k_active<<<dim3(TN * TN / 256, S), 256, 0, g.st>>>(g.d_tab, sp->ta, g.d_act, g.d_nact, nullptr);
+        k_active<<<dim3(TN / ROW_WARPS, S), 32 * ROW_WARPS, 0, g.st>>>(g.d_tab, sp->ta, g.d_act, g.d_nact, nullptr);
         k_scan<<<dim3(SCAN_BLOCKS, S), 256, 0, g.st>>>(g.d_tab, g.d_act, g.d_nact, g.d_ibT, g.d_ibC, g.d_loT, g.d_hiT, *sp, g.sc, g.d_out, g.d_ncand, cap,
                                                        nullptr);
     }
@@ -388,7 +401,7 @@ int scan_seeds_device(const SeedNoise *noise, const uint32_t *n_dev, uint32_t ca
     // a wave fills a third or less of its seed capacity: the grids stride over the counted seeds instead of
     // covering the capacity with blocks that would only return
     const uint32_t ys = std::min(cap_seeds, 128u);
-    k_active<<<dim3(TN * TN / 256, ys), 256, 0, st>>>(tab, sp.ta, act, nact, n_dev);
+    k_active<<<dim3(TN / ROW_WARPS, ys), 32 * ROW_WARPS, 0, st>>>(tab, sp.ta, act, nact, n_dev);
     k_scan<<<dim3(SCAN_BLOCKS, ys), 256, 0, st>>>(tab, act, nact, g.d_ibT, g.d_ibC, g.d_loT, g.d_hiT, sp, g.sc,
                                                          reinterpret_cast<Cand *>(cand), ncand, cap, n_dev);
     DSG_CU(cudaGetLastError());
