@@ -115,6 +115,7 @@ struct State {
     Oct *d_oct = nullptr;
     uint64_t *h_s3 = nullptr; float *h_a3 = nullptr;
     int pg_blocks = 0, fg_blocks = 0;
+    SplitMax *d_split = nullptr;                             // the full gate's split seeds
 };
 State &S() { static State s; return s; }
 
@@ -131,6 +132,9 @@ void setup_locked(State &g) {
     g.pg_blocks = std::max(1, occ) * device_info().sms;
     DSG_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fullgate, FG_THREADS, 0));
     g.fg_blocks = std::max(1, occ) * device_info().sms;
+    DSG_CU(cudaMalloc(&g.d_split, size_t(g.fg_blocks / FG_SPLIT + 1) * sizeof(SplitMax)));
+    DSG_CU(cudaMemsetAsync(g.d_split, 0, size_t(g.fg_blocks / FG_SPLIT + 1) * sizeof(SplitMax), g.st));
+    DSG_CU(cudaStreamSynchronize(g.st));                     // the batches may run on other streams
     g.ready = true;
 }
 void ensure_buffers(State &g, uint64_t batch) {
@@ -160,7 +164,7 @@ void enqueue_batch(State &g, cudaStream_t st, uint64_t start, uint64_t nb, const
     k_phase<<<pb, 256, 0, st>>>(start, nb, double(c.maxph), g.d_s1, g.d_n, g.cap1);
     k_octinit<<<unsigned(device_info().sms) * 13, OCT_THREADS, 0, st>>>(g.d_s1, g.d_n, g.cap1, g.d_oct);
     k_amp256<AMP_AA><<<g.pg_blocks, PG_THREADS, 0, st>>>(g.d_oct, g.d_s1, g.d_n, g.cap1, c.pthr, g.t256, g.d_s2, g.d_idx2, g.d_n + 1, g.cap2, nullptr);
-    k_fullgate<<<g.fg_blocks, FG_THREADS, 0, st>>>(g.d_oct, g.d_s2, g.d_idx2, g.d_n + 1, g.cap2, c.amp, g.t512, g.d_s3, g.d_a3, g.d_n + 2, g.cap3, nullptr);
+    k_fullgate<<<g.fg_blocks, FG_THREADS, 0, st>>>(g.d_oct, g.d_s2, g.d_idx2, g.d_n + 1, g.cap2, c.amp, g.t512, g.d_s3, g.d_a3, g.d_n + 2, g.cap3, nullptr, g.d_split);
     DSG_CU(cudaGetLastError());
 }
 // A gate with buffers of its own, for the device-resident searcher: batches of up to `batch` indices enqueued
@@ -179,6 +183,7 @@ void lane_destroy(Lane *l) {
     State &g = l->g;
     cudaFree(g.d_s1); cudaFree(g.d_s2); cudaFree(g.d_s3); cudaFree(g.d_idx2); cudaFree(g.d_a3); cudaFree(g.d_oct); cudaFree(g.d_n);
     cudaFreeHost(g.h_n); cudaFreeHost(g.h_s3); cudaFreeHost(g.h_a3);
+    cudaFree(g.d_split);
     if (g.st) cudaStreamDestroy(g.st);
     delete l;
 }
@@ -230,7 +235,7 @@ extern "C" int dsg_gate_amps(const uint64_t *seeds, uint32_t n, float *pre, floa
         DSG_CU(cudaMemcpy(d_n, hn, 16, cudaMemcpyHostToDevice));
         k_octinit<<<(2 * n + OCT_THREADS - 1) / OCT_THREADS, OCT_THREADS>>>(d_s, d_n, n, d_oct);
         k_amp256<AMP_AA><<<g.pg_blocks, PG_THREADS>>>(d_oct, d_s, d_n, n, -1e30, g.t256, d_o, d_i, d_n + 1, n, d_pre);
-        k_fullgate<<<g.fg_blocks, FG_THREADS>>>(d_oct, d_s, nullptr, d_n + 2, n, -1e30f, g.t512, d_o, d_a, d_n + 3, n, d_full);
+        k_fullgate<<<g.fg_blocks, FG_THREADS>>>(d_oct, d_s, nullptr, d_n + 2, n, -1e30f, g.t512, d_o, d_a, d_n + 3, n, d_full, nullptr);
         DSG_CU(cudaGetLastError());
         DSG_CU(cudaMemcpy(pre, d_pre, size_t(n) * 8, cudaMemcpyDeviceToHost));
         DSG_CU(cudaMemcpy(full, d_full, size_t(n) * 8, cudaMemcpyDeviceToHost));
@@ -371,7 +376,7 @@ extern "C" int dsg_gate_onepar_run(uint64_t start, uint64_t count, const dsg_gat
             k_octinit<<<unsigned(device_info().sms) * 13, OCT_THREADS, 0, st>>>(g.d_s1, g.d_n, g.cap1, g.d_oct);
             k_amp256<AMP_ONEPAR><<<blocks, PG_THREADS, 0, st>>>(g.d_oct, g.d_s1, g.d_n, g.cap1, thr, g.t256, g.d_s2, g.d_idx2, g.d_n + 1, g.cap2, nullptr);
             k_fullgate<<<g.fg_blocks, FG_THREADS, 0, st>>>(g.d_oct, g.d_s2, g.d_idx2, g.d_n + 1, g.cap2, cfg->amp, g.t512, g.d_s3, g.d_a3, g.d_n + 2,
-                                                          g.cap3, nullptr);
+                                                          g.cap3, nullptr, g.d_split);
             DSG_CU(cudaGetLastError());
             DSG_CU(cudaMemcpyAsync(g.h_n, g.d_n, 16, cudaMemcpyDeviceToHost, st));
             DSG_CU(cudaStreamSynchronize(st));
@@ -491,7 +496,7 @@ extern "C" int dsg_gate_bench(uint64_t start, uint64_t per_step, uint32_t steps,
             if (timed) DSG_CU(cudaEventRecord(ev[4 + 5 * k], g.st));
             k_amp256<AMP_AA><<<g.pg_blocks, PG_THREADS, 0, g.st>>>(g.d_oct, g.d_s1, g.d_n, g.cap1, c.pthr, g.t256, g.d_s2, g.d_idx2, g.d_n + 1, g.cap2, nullptr);
             if (timed) DSG_CU(cudaEventRecord(ev[5 + 5 * k], g.st));
-            k_fullgate<<<g.fg_blocks, FG_THREADS, 0, g.st>>>(g.d_oct, g.d_s2, g.d_idx2, g.d_n + 1, g.cap2, c.amp, g.t512, g.d_s3, g.d_a3, g.d_n + 2, g.cap3, nullptr);
+            k_fullgate<<<g.fg_blocks, FG_THREADS, 0, g.st>>>(g.d_oct, g.d_s2, g.d_idx2, g.d_n + 1, g.cap2, c.amp, g.t512, g.d_s3, g.d_a3, g.d_n + 2, g.cap3, nullptr, g.d_split);
             if (timed) DSG_CU(cudaEventRecord(ev[6 + 5 * k], g.st));
             DSG_CU(cudaGetLastError());
             DSG_CU(cudaMemcpyAsync(h_cnt + 4 * it, g.d_n, 16, cudaMemcpyDeviceToHost, g.st));
@@ -523,7 +528,7 @@ void launch_amps_on(const uint64_t *d_seeds, uint32_t n, void *d_oct, uint32_t *
     Oct *oct = static_cast<Oct *>(d_oct);
     k_octinit<<<(2 * n + OCT_THREADS - 1) / OCT_THREADS, OCT_THREADS, 0, st>>>(d_seeds, d_counters, n, oct);
     k_amp256<AMP_AA><<<pg_blocks, PG_THREADS, 0, st>>>(oct, d_seeds, d_counters, n, -1e30, t256, d_tmp_seeds, d_tmp_idx, d_counters + 1, n, d_pre);
-    k_fullgate<<<fg_blocks, FG_THREADS, 0, st>>>(oct, d_seeds, nullptr, d_counters + 2, n, -1e30f, t512, d_tmp_seeds, d_tmp_amp, d_counters + 3, n, d_full);
+    k_fullgate<<<fg_blocks, FG_THREADS, 0, st>>>(oct, d_seeds, nullptr, d_counters + 2, n, -1e30f, t512, d_tmp_seeds, d_tmp_amp, d_counters + 3, n, d_full, nullptr);
 }
 size_t oct_bytes() { return sizeof(Oct); }
 int pregate_blocks_per_sm() { int occ = 0; cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_amp256<AMP_AA>, PG_THREADS, 0); return occ; }

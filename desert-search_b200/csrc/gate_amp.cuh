@@ -486,11 +486,20 @@ __device__ __forceinline__ float exact_cell512(const Side512 &sd, float *__restr
     return __fmul_rn(o, tp.norm);
 }
 
+// Maxima of a seed whose columns are split over CTAs (floats in unsigned order) and the CTAs that have added theirs; all
+// zero between launches.
+struct SplitMax { uint32_t top[2], arrived, pad; };
+__device__ __forceinline__ uint32_t order_float(float v) { const uint32_t b = __float_as_uint(v); return b >> 31 ? ~b : b | 0x80000000u; }
+__device__ __forceinline__ float unorder_float(uint32_t o) { return __uint_as_float(o >> 31 ? o & 0x7fffffffu : ~o); }
+constexpr int FG_SPLIT = 4;
 // One CTA per seed; a warp holds FG_ZL rows per lane of one side and row parity (rows 2 (lane + 32 q) + parity).
+// A launch of few seeds takes the time of one (about 90 us, one SM's work).  While FG_SPLIT CTAs per seed fit the grid,
+// each therefore takes a quarter of the columns (and the blur's run-in before them), evaluates its own exact cells,
+// and the last to arrive decides: 47 seeds 100 -> 60 us.  split (may be null: never split) holds gridDim.x / FG_SPLIT entries.
 __global__ void __launch_bounds__(FG_THREADS, DSG_FG_MINBLOCKS)
 k_fullgate(const Oct *__restrict__ oct, const uint64_t *__restrict__ seeds, const uint32_t *__restrict__ idx, const uint32_t *__restrict__ n_in,
            uint32_t cap_in, float thr, const __grid_constant__ Taps512 tp, uint64_t *__restrict__ out_seed, float *__restrict__ out_amp,
-           uint32_t *__restrict__ n_out, uint32_t cap_out, float *__restrict__ side_amp) {
+           uint32_t *__restrict__ n_out, uint32_t cap_out, float *__restrict__ side_amp, SplitMax *__restrict__ split) {
     constexpr int W = 2 * FG_WARPS;                             // warps per side
     __shared__ __align__(16) Side512 sides[2];
     __shared__ float sTop[2][2 * W], sAmp[2 * W];
@@ -500,7 +509,11 @@ k_fullgate(const Oct *__restrict__ oct, const uint64_t *__restrict__ seeds, cons
     const uint32_t n = min(*n_in, cap_in);
     const float floor0 = thr > 0.4f ? 0.44f * thr : AMP_FLOOR;
     int it = 0;
-    for (uint32_t s = blockIdx.x; s < n; s += gridDim.x) {
+    const bool parts = split && n * FG_SPLIT <= gridDim.x;       // n is at most the survivor capacity: no overflow
+    for (uint32_t unit = blockIdx.x; unit < (parts ? n * FG_SPLIT : n); unit += gridDim.x) {
+        const uint32_t s = parts ? unit / FG_SPLIT : unit;
+        // lattice columns: the run-in from jb, cells from jb + 7 to je - 1
+        const int jb = parts ? 1 + int(unit % FG_SPLIT) * (256 / FG_SPLIT) : 1, je = parts ? jb + 7 + 256 / FG_SPLIT : FG_COLS;
         const Oct &p = oct[2 * size_t(idx ? idx[s] : s) + side];
         __syncthreads();                                         // the previous seed's cells are done with the shared arrays
         if (t < 16) reinterpret_cast<uint4 *>(sd.P)[t] = reinterpret_cast<const uint4 *>(p.perm)[t];
@@ -553,7 +566,7 @@ k_fullgate(const Oct *__restrict__ oct, const uint64_t *__restrict__ seeds, cons
         __syncthreads();
         const int row0 = lane + 32 * FG_ZL * zh;
         const char *uv0 = reinterpret_cast<const char *>(&sd.a.uv[pz][0][row0]), *uv1 = reinterpret_cast<const char *>(&sd.a.uv[pz][1][row0]);
-        float start = floor0;
+        float start = parts ? -1e9f : floor0;                    // a part cannot drop the seed: it lists without a floor
         for (;;) {
             Run r{-1e9f, start, 0};
             float acc[2][FG_ZL], pend[14][FG_ZL];                // pend: a ring, as in k_amp256, two steps per column
@@ -570,17 +583,17 @@ k_fullgate(const Oct *__restrict__ oct, const uint64_t *__restrict__ seeds, cons
             };
             {
                 float U[FG_ZL], V[FG_ZL];
-                column(0, U, V);
+                column(jb - 1, U, V);
                 #pragma unroll
                 for (int h = 0; h < 2; h++)
                     #pragma unroll
                     for (int q = 0; q < FG_ZL; q++) acc[h][q] = __fmaf_rn(a[h][0], U[q], b[h][0] * V[q]);
             }
             #pragma unroll 1
-            for (int J0 = 1; J0 < FG_COLS; J0 += 7) {
+            for (int J0 = jb; J0 < je; J0 += 7) {
                 #pragma unroll
                 for (int ph = 0; ph < 7; ph++) {
-                    if (ph == (FG_COLS - 1) % 7 && J0 + ph == FG_COLS) break;
+                    if ((ph == (FG_COLS - 1) % 7 || ph == (7 + 256 / FG_SPLIT) % 7) && J0 + ph == je) break;
                     float U[FG_ZL], V[FG_ZL];
                     column(J0 + ph, U, V);
                     // column J completes samples 2 J - 2 - dx0 and the next: two blur steps
@@ -600,7 +613,7 @@ k_fullgate(const Oct *__restrict__ oct, const uint64_t *__restrict__ seeds, cons
                         float mx = c.v[0];
                         #pragma unroll
                         for (int q = 1; q < FG_ZL; q++) mx = fmaxf(mx, c.v[q]);
-                        if (__any_sync(0xffffffffu, mx > r.lim) && J0 + ph >= 8)
+                        if (__any_sync(0xffffffffu, mx > r.lim) && J0 + ph >= jb + 7)
                             r = list_cells<FG_ZL>(c, uint32_t((2 * (J0 + ph) - 9 - dx0 + h) & 511) << 9 | uint32_t(2 * row0 + pz), 64u, &sd.list[wi], r, lane);
                     }
                 }
@@ -614,13 +627,13 @@ k_fullgate(const Oct *__restrict__ oct, const uint64_t *__restrict__ seeds, cons
             #pragma unroll
             for (int k = 0; k < 2 * W; k++) top[k / W] = fmaxf(top[k / W], sTop[par][k]);
             const float ok = start + AMP_E2;                     // as in k_amp256
-            if (double(fmaxf(top[0], ok)) + double(fmaxf(top[1], ok)) + double(AMP_E2) < double(thr)) break;
+            if (!parts && double(fmaxf(top[0], ok)) + double(fmaxf(top[1], ok)) + double(AMP_E2) < double(thr)) break;
             if (top[0] < ok || top[1] < ok) { start = -1e9f; continue; }
             corner_tables512(p, tp.w, sd.x.tab, t);
             __syncthreads();
             const float cut = top[side] - AMP_E2;
             float m = -1e9f;
-            const bool every = nl > AMP_CAP;                     // this warp's cells: columns x the rows of its lanes
+            const bool every = nl > AMP_CAP;                     // this warp's cells: columns (a part: all of them) x the rows of its lanes
             for (int c = 0; c < (every ? 512 * 32 * FG_ZL : nl); c++) {
                 if (!every && sd.list[wi].val[c] < cut) continue;
                 const uint32_t pos = every ? uint32_t(c / (32 * FG_ZL)) << 9 | uint32_t(2 * (c % (32 * FG_ZL) + 32 * FG_ZL * zh) + pz) : sd.list[wi].pos[c];
@@ -632,6 +645,15 @@ k_fullgate(const Oct *__restrict__ oct, const uint64_t *__restrict__ seeds, cons
                 float ma = -1e9f, mb = -1e9f;
                 #pragma unroll
                 for (int k = 0; k < W; k++) { ma = fmaxf(ma, sAmp[k]); mb = fmaxf(mb, sAmp[W + k]); }
+                if (parts) {
+                    SplitMax &x = split[s];
+                    atomicMax(&x.top[0], order_float(ma)); atomicMax(&x.top[1], order_float(mb));
+                    __threadfence();
+                    if (atomicAdd(&x.arrived, 1u) != FG_SPLIT - 1) break;
+                    __threadfence();
+                    ma = unorder_float(atomicExch(&x.top[0], 0u)); mb = unorder_float(atomicExch(&x.top[1], 0u));
+                    x.arrived = 0;
+                }
                 const float amp = __fadd_rn(ma, mb);
                 if (side_amp) { side_amp[2 * size_t(s)] = ma; side_amp[2 * size_t(s) + 1] = mb; }
                 if (amp >= thr) {
