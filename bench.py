@@ -48,13 +48,13 @@ UNIT = "gated seeds/s"
 START = 2 * 10**13
 PER_STEP = 1 << 24
 RANK_STRIDE = 10**12            # per-GPU seed ranges, as deploy/prun.sh assigns them
-# pre-gate: 2 sides x 256^2 cells x 18 corner-table gathers of 4 bytes per phase-passed seed
-PRE_BYTES_PER_SEED = 2 * 256 * 256 * 18 * 4
+# pre-gate screen: 2 sides x 256 rows x 267 lattice columns x 16 bytes of sequence values (two hashes) per phase-passed seed
+PRE_BYTES_PER_SEED = 2 * 256 * 267 * 16
 SMEM_BYTES_PER_CLK_PER_SM = 128  # 32 banks x 4 bytes
 FP64_FLOPS_PER_CLK_PER_SM = 128  # 64 FP64 FMA lanes per SM (B200) x 2 flops
-# k_pregate DRAM traffic per phase-passed seed from one ncu capture (dram__bytes_read.sum + write.sum =
-# 150.5 MB + 6.1 MB over 241,519 seeds on 2^25 seed indices): the seed's octave table read once
-PRE_DRAM_BYTES_PER_SEED = (150.5e6 + 6.1e6) / 241519
+# k_amp256 DRAM traffic per phase-passed seed from one ncu capture (dram__bytes_read.sum + write.sum =
+# 37.0 MB + 0.1 MB over 60,230 seeds on 2^23 seed indices): the seed's octave table read once
+PRE_DRAM_BYTES_PER_SEED = (37.0e6 + 0.1e6) / 60230
 # k_tile_eval FP64 work per evaluated cell: executed DADD + DMUL + 2 x DFMA (ncu counters over every k_tile_eval
 # launch) divided by the cells of the evaluated 16x16 sub-blocks, on exact step-1 floods of the 32 largest verified
 # finds (2,297 on step-8 floods of the 6 largest).  Counted with each gradient as one DADD, the reference's
@@ -191,8 +191,8 @@ def search_steps(dsgpu, base, steps, warmup, per_step):
 
 # ---------------------------------------------------------------------------- the gate alone
 def gate_leg(dsgpu, sm_mhz, sms, steps=6, warmup=3):
-    """The seed gate (y-phase, octave init, pre-gate, full gate) alone on 2^26 indices per step, its k_pregate
-    against the shared-memory gather roofline, and the reference's tgate (its GPU gate) on the same seeds."""
+    """The seed gate (y-phase, octave init, pre-gate, full gate) alone on 2^26 indices per step, its pre-gate
+    kernel (k_amp256) against the shared-memory roofline, and the reference's tgate (its GPU gate) on the same seeds."""
     n = 1 << 26
     ms, mk, counts = dsgpu.gate_bench(START, n, steps, warmup)
     pre_ms = float(mk[2])
@@ -201,9 +201,9 @@ def gate_leg(dsgpu, sm_mhz, sms, steps=6, warmup=3):
     out = {"seeds_per_step": n, "steps": steps, "gated_per_s": counts[3] / (ms / 1e3), "seeds_per_s": counts[0] / (ms / 1e3),
            "kernel_ms": {"phase": float(mk[0]), "octave_init": float(mk[1]), "pregate": pre_ms, "fullgate": float(mk[3])},
            "counts": {"seeds": int(counts[0]), "phase_passed": int(counts[1]), "pre_passed": int(counts[2]), "gated": int(counts[3])},
-           "roofline": {"bound": "smem", "kernel": "k_pregate", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+           "roofline": {"bound": "smem", "kernel": "k_amp256", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                         "traffic": counts[1] / steps * PRE_DRAM_BYTES_PER_SEED,
-                        "note": "shared-memory gather bytes (18 corner-table words per cell) / k_pregate event time; peak = SMs x 128 B/clk "
+                        "note": "shared-memory bytes of the screen (16 per cell and lattice column) / k_amp256 event time; peak = SMs x 128 B/clk "
                                 "at the median sampled SM clock; traffic = DRAM bytes per launch scaled from an ncu capture"}}
     tg = ref_exe("tgate")
     if tg:
@@ -579,7 +579,7 @@ def run_ours(args):
         gate = gate_leg(dsgpu, sm_mhz, sms)
         out["gate"] = gate
         out["roofline"] = dict(gate["roofline"])
-        out["roofline"]["scope"] = "k_pregate, the gate's dominant kernel, timed in the gate leg on the same seed stream"
+        out["roofline"]["scope"] = "k_amp256, the gate's dominant kernel, timed in the gate leg on the same seed stream"
         out["cpu_baseline"] = cpu_baseline(os.cpu_count() or 1)
         if not args.no_extras:
             out["pipeline"], cands = searcher_runs()
