@@ -518,48 +518,76 @@ __global__ void __launch_bounds__(256) k_cover_pairs(const Hot *__restrict__ hot
         }
     }
 }
-// Warp per seed: the reference's walk over its sites in rank order (dsearch_desert.cpp:326-372): a hot site is
+// Block per seed: the reference's walk over its sites in rank order (dsearch_desert.cpp:326-372): a hot site is
 // skipped when a flood used so far covers it (lane j < CW holds word j of the used set); else its flood is used,
 // and a big one (hot area >= hot_min) becomes a proxy zone of 32-quart cells around the step-128 flood's bbox.
-__global__ void __launch_bounds__(256) k_cover(const Hot *__restrict__ hot, const uint32_t *__restrict__ nsites, const int32_t *__restrict__ f1,
+// What bounds it is the latency of one seed, however few seeds there are.  Only "is it covered" depends on the sites
+// before, so a thread per site looks at the rest (hot, small, area) and the block brings the matrix to shared memory;
+// the first warp's walk then touches no global memory.  (A warp per seed that read each site's data in turn: 21 seeds of
+// 236 sites 285 us, 34 now.)
+constexpr int COVER_THREADS = int(CW) * 32;
+static_assert(COVER_THREADS >= int(MS), "a thread per site");
+__global__ void __launch_bounds__(COVER_THREADS) k_cover(const Hot *__restrict__ hot, const uint32_t *__restrict__ nsites, const int32_t *__restrict__ f1,
                                                const int32_t *__restrict__ f2, const FloodStat *__restrict__ st1, const FloodStat *__restrict__ st2,
                                                Params P, const uint32_t *__restrict__ cvm, uint32_t *__restrict__ nzone, DZone *__restrict__ zslot,
                                                ZoneMeta *__restrict__ zmeta, uint32_t *ctr) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    __shared__ uint32_t rows[MS * CW], s_on[CW], s_big[CW], s_walked[CW];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t s = blockIdx.x;
     if (s >= ctr[C_NS]) return;
-    uint32_t used = 0;                                   // word `lane` of the used set (lanes < CW)
-    uint32_t nz = 0, nhot = 0, nbig = 0;
-    const uint32_t ns = nsites[s];
-    for (uint32_t r = 0; r < ns; r++) {
-        const uint32_t w = s * MS + r;
-        const Hot h = hot[w];
-        if (h.bt < 0.55) continue;
-        const uint32_t words = (r + 31) >> 5;            // bits of sites before r
-        const bool hit = uint32_t(lane) < words && (used & cvm[size_t(w) * CW + lane]) != 0;
-        if (__any_sync(0xffffffffu, hit)) continue;
-        if (uint32_t(lane) == (r >> 5)) used |= 1u << (r & 31);
-        nhot++;
-        const int32_t k1 = f1[w];
-        if (small_zone(st1[k1], P)) continue;
-        const FloodStat a = st2[f2[w]];
-        const double hot_area = double(a.cells) * 128.0 * 128 * 16 / 1e6;
-        if (hot_area < P.hot_min) continue;
-        nbig++;
-        if (lane == 0) {
-            DZone z{};
-            z.x0 = int(floor((a.minx - 128) / 32.0)) * 32; z.z0 = int(floor((a.minz - 128) / 32.0)) * 32;
-            z.nx = (a.maxx + 128 - z.x0) / 32 + 1; z.nz = (a.maxz + 128 - z.z0) / 32 + 1;
-            z.seed = int32_t(s);
-            zslot[size_t(s) * ZPS + nz] = z;
-            zmeta[size_t(s) * ZPS + nz] = {s, r, hot_area};
+    const uint32_t ns = nsites[s], r0 = threadIdx.x;
+    const size_t w0 = size_t(s) * MS;
+    for (uint32_t k = threadIdx.x; k < ns * CW; k += COVER_THREADS) rows[k] = cvm[w0 * CW + k];
+    bool on = false, big = false;
+    FloodStat a{};
+    double hot_area = 0;
+    if (r0 < ns) {
+        on = !(hot[w0 + r0].bt < 0.55);
+        const int32_t k1 = f1[w0 + r0], k2 = f2[w0 + r0];    // -1 where there is no such flood: not hot, or small
+        if (k2 >= 0) a = st2[k2];
+        if (on && !small_zone(st1[k1], P)) {
+            hot_area = double(a.cells) * 128.0 * 128 * 16 / 1e6;
+            big = !(hot_area < P.hot_min);
         }
-        nz++;
     }
-    if (lane == 0) {
+    const uint32_t ons = __ballot_sync(0xffffffffu, on), bigs = __ballot_sync(0xffffffffu, big);
+    if (lane == 0) { s_on[warp] = ons; s_big[warp] = bigs; }
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t used = 0;                                   // word `lane` of the used set (lanes < CW)
+        for (uint32_t v = 0; v < CW; v++) {
+            uint32_t walked = 0;                             // the sites whose flood is used
+            for (uint32_t m = s_on[v]; m; m &= m - 1) {
+                const uint32_t b = uint32_t(__ffs(m) - 1), r = 32 * v + b;
+                const uint32_t words = (r + 31) >> 5;        // bits of sites before r
+                const bool hit = uint32_t(lane) < words && (used & rows[r * CW + lane]) != 0;
+                if (__any_sync(0xffffffffu, hit)) continue;
+                if (uint32_t(lane) == v) used |= 1u << b;
+                walked |= 1u << b;
+            }
+            if (lane == 0) s_walked[v] = walked;
+        }
+    }
+    __syncthreads();
+    const uint32_t zs = s_walked[warp] & bigs;
+    uint32_t at = uint32_t(__popc(zs & ((1u << lane) - 1))), nz = 0, nhot = 0;
+    for (int v = 0; v < int(CW); v++) {
+        const uint32_t n = uint32_t(__popc(s_walked[v] & s_big[v]));
+        at += v < warp ? n : 0;
+        nz += n; nhot += uint32_t(__popc(s_walked[v]));
+    }
+    if (zs >> lane & 1) {
+        DZone z{};
+        z.x0 = int(floor((a.minx - 128) / 32.0)) * 32; z.z0 = int(floor((a.minz - 128) / 32.0)) * 32;
+        z.nx = (a.maxx + 128 - z.x0) / 32 + 1; z.nz = (a.maxz + 128 - z.z0) / 32 + 1;
+        z.seed = int32_t(s);
+        zslot[size_t(s) * ZPS + at] = z;
+        zmeta[size_t(s) * ZPS + at] = {s, r0, hot_area};
+    }
+    if (threadIdx.x == 0) {
         nzone[s] = nz;
-        atomicAdd(ctr + C_NHOT, nhot); atomicAdd(ctr + C_NBIG, nbig);
-        atomicMax(ctr + C_MAXZ, nbig);
+        atomicAdd(ctr + C_NHOT, nhot); atomicAdd(ctr + C_NBIG, nz);
+        atomicMax(ctr + C_MAXZ, nz);
     }
 }
 // One block: the seeds' zones concatenated in seed order (zfirst[s] = first zone of seed s), their cell offsets
@@ -671,70 +699,85 @@ __global__ void __launch_bounds__(256) k_comp_order(const dsg_component *__restr
         }
     }
 }
-// Warp per seed: components of its zones in (zone, first cell) order, each new one (by its smallest column and
+// Block per seed: components of its zones in (zone, first cell) order, each new one (by its smallest column and
 // row) an evaluation whose start is the interior cell nearest the centroid (alternatives at ranks n/3, 2n/3);
-// each with its sort key (cells, index) for k_eval_order.  The lanes load 32 components at a time; the signatures
-// seen live in shared memory.
-constexpr int EV_WARPS = 4;
-constexpr size_t EV_SMEM = size_t(EV_WARPS) * EVC * 8;
-__global__ void __launch_bounds__(EV_WARPS * 32) k_evals(const uint32_t *__restrict__ zfirst, const DZone *__restrict__ zones,
+// each with its sort key (cells, index) for k_eval_order.  The seed's components are one run of zcomp, taken a block's
+// width at a time: a hash table of the signatures in shared memory keeps each signature's first component, and a
+// component that is the first of its signature takes the next place.  (A warp per seed comparing one component after
+// another with all signatures before it took the time of the seed with most components, whatever the wave: 21 seeds, 164
+// evaluations at most, 119 us, 7 now.)
+constexpr int EV_THREADS = 256;
+constexpr uint32_t EV_SLOTS = 4096;          // at most EVC + EV_THREADS signatures before a full seed stops: always a free slot
+static_assert(EV_SLOTS > EVC + EV_THREADS && (EV_SLOTS & (EV_SLOTS - 1)) == 0, "the table never fills");
+constexpr size_t EV_SMEM = size_t(EV_SLOTS) * (8 + 4);
+constexpr unsigned long long EV_FREE = 1ull << 63;   // x = -2^31: no quart of the world
+__global__ void __launch_bounds__(EV_THREADS) k_evals(const uint32_t *__restrict__ zfirst, const DZone *__restrict__ zones,
                                                          const ZoneMeta *__restrict__ zmeta, const uint32_t *__restrict__ zoff,
                                                          const uint32_t *__restrict__ zcomp, const dsg_component *__restrict__ rec, Params P,
                                                          Eval *__restrict__ evu, unsigned long long *__restrict__ ekey,
                                                          uint32_t *__restrict__ nev, uint32_t *ctr) {
     extern __shared__ __align__(16) unsigned char ev_smem[];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int64_t *seen = reinterpret_cast<int64_t *>(ev_smem) + size_t(w) * EVC;
-    const uint32_t s = blockIdx.x * EV_WARPS + w;
+    __shared__ uint32_t s_cnt[EV_THREADS / 32];
+    unsigned long long *sig = reinterpret_cast<unsigned long long *>(ev_smem);
+    uint32_t *first = reinterpret_cast<uint32_t *>(sig + EV_SLOTS);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t s = blockIdx.x;
     if (s >= ctr[C_NS]) return;
     Eval *U = evu + size_t(s) * EVC;
     unsigned long long *K = ekey + size_t(s) * EVC;
-    uint32_t ne = 0;                                     // evaluations so far (= signatures seen), uniform across the warp
-    bool full = false;
     const uint32_t nzw = ctr[C_ZONES];
-    for (uint32_t zi = zfirst[s]; zi < zfirst[s + 1] && zi < nzw; zi++) {
-        const DZone z = zones[zi];
-        const ZoneMeta m = zmeta[zi];
-        const uint32_t *L = zcomp + zoff[zi];
-        const uint32_t nc = zoff[zi + 1] - zoff[zi];
-        for (uint32_t i0 = 0; i0 < nc; i0 += 32) {
-            dsg_component c{};
-            int elig = 0;
-            int64_t sg = 0;
-            if (i0 + lane < nc) {
-                c = rec[L[i0 + lane]];
-                elig = c.cells * 32.0 * 32 * 16 / 1e6 >= 1;
-                sg = (int64_t(z.x0 + c.minx * 32) << 32) | uint32_t(z.z0 + c.minz * 32);
+    const uint32_t begin = zoff[min(zfirst[s], nzw)], end = zoff[min(zfirst[s + 1], nzw)];
+    if (begin < end)
+        for (uint32_t k = threadIdx.x; k < EV_SLOTS; k += EV_THREADS) { sig[k] = EV_FREE; first[k] = ~0u; }
+    __syncthreads();
+    uint32_t ne = 0;                                     // evaluations so far (= signatures seen), uniform across the block
+    for (uint32_t i0 = begin; i0 < end && ne <= EVC; i0 += EV_THREADS) {
+        const uint32_t i = i0 + threadIdx.x;
+        dsg_component c{};
+        DZone z{};
+        bool elig = false;
+        uint32_t slot = 0;
+        if (i < end) {
+            c = rec[zcomp[i]];
+            z = zones[c.zone];
+            elig = c.cells * 32.0 * 32 * 16 / 1e6 >= 1;
+        }
+        if (elig) {
+            const unsigned long long g = uint64_t(uint32_t(z.x0 + c.minx * 32)) << 32 | uint32_t(z.z0 + c.minz * 32);
+            slot = uint32_t(g * 0x9e3779b97f4a7c15ull >> 40) & (EV_SLOTS - 1);
+            for (;; slot = (slot + 1) & (EV_SLOTS - 1)) {
+                const unsigned long long was = atomicCAS(&sig[slot], EV_FREE, g);
+                if (was == EV_FREE || was == g) break;
             }
-            const uint32_t cnt = min(32u, nc - i0);
-            for (uint32_t j = 0; j < cnt; j++) {
-                if (!__shfl_sync(0xffffffffu, elig, j)) continue;
-                const int64_t sj = __shfl_sync(0xffffffffu, sg, j);
-                bool dup = false;
-                for (uint32_t k = lane; k < ne; k += 32) dup |= seen[k] == sj;
-                if (__any_sync(0xffffffffu, dup)) continue;
-                if (ne == EVC) { full = true; continue; }
-                if (uint32_t(lane) == j) {                   // the component's own lane writes its evaluation
-                    seen[ne] = sj;
-                    K[ne] = (uint64_t(c.cells) << 32) | ne;
-                    const int32_t cell = c.inner ? c.pick[0] : c.first;
-                    Eval e{};
-                    e.rank = m.rank; e.x = z.x0 + (cell % z.nx) * 32; e.z = z.z0 + (cell / z.nx) * 32;
-                    e.proxy = c.cells * 32.0 * 32 * 16 / 1e6; e.s8 = -1; e.s4 = 0; e.hot = m.hot;
-                    e.nalt = c.inner ? 2 : 0;
-                    for (int a = 0; a < e.nalt; a++) { e.ax[a] = z.x0 + (c.pick[a + 1] % z.nx) * 32; e.az[a] = z.z0 + (c.pick[a + 1] / z.nx) * 32; }
-                    U[ne] = e;
-                }
-                ne++;
-                __syncwarp();
-            }
+            atomicMin(&first[slot], i);
+        }
+        __syncthreads();
+        const bool fresh = elig && first[slot] == i;
+        const uint32_t m = __ballot_sync(0xffffffffu, fresh);
+        if (lane == 0) s_cnt[warp] = uint32_t(__popc(m));
+        __syncthreads();
+        uint32_t at = ne + __popc(m & ((1u << lane) - 1));
+        #pragma unroll
+        for (int k = 0; k < EV_THREADS / 32; k++) { at += k < warp ? s_cnt[k] : 0; ne += s_cnt[k]; }
+        if (fresh && at < EVC) {
+            const ZoneMeta mt = zmeta[c.zone];
+            K[at] = (uint64_t(c.cells) << 32) | at;
+            const int32_t cell = c.inner ? c.pick[0] : c.first;
+            Eval e{};
+            e.rank = mt.rank; e.x = z.x0 + (cell % z.nx) * 32; e.z = z.z0 + (cell / z.nx) * 32;
+            e.proxy = c.cells * 32.0 * 32 * 16 / 1e6; e.s8 = -1; e.s4 = 0; e.hot = mt.hot;
+            e.nalt = c.inner ? 2 : 0;
+            #pragma unroll
+            for (int a = 0; a < 2; a++)
+                if (c.inner) { e.ax[a] = z.x0 + (c.pick[a + 1] % z.nx) * 32; e.az[a] = z.z0 + (c.pick[a + 1] / z.nx) * 32; }
+            U[at] = e;
         }
     }
-    if (lane == 0) {
-        if (full) atomicOr(ctr + C_FLAGS, F_EVALS);
-        atomicMax(ctr + C_MAXEV, ne + (full ? 1 : 0));
+    if (threadIdx.x == 0) {
+        if (ne > EVC) { atomicOr(ctr + C_FLAGS, F_EVALS); ne = EVC + 1; }
+        atomicMax(ctr + C_MAXEV, ne);
         if (s == 0 && ctr[C_PROXY + 3]) atomicOr(ctr + C_FLAGS, F_LABEL);
-        nev[s] = ne;
+        nev[s] = min(ne, EVC);
     }
 }
 // Block per seed: std::sort(ev, proxy descending) with the library's permutation, computed by the block
@@ -831,42 +874,57 @@ __global__ void k_retry(const Try *__restrict__ tries, const int32_t *__restrict
         }
     }
 }
-// Thread per seed: step-4 areas, the seed's best exact area, its seeds.csv record and its CSV rows.
-__global__ void k_results(const uint64_t *__restrict__ seeds, const SeedNoise *__restrict__ noise, const float *__restrict__ mx,
+// Warp per seed: step-4 areas, the seed's best exact area, its seeds.csv record and its CSV rows.  (A thread per seed
+// waited for each of the seed's evaluations in turn: 63 us for 21 seeds, 10 now.)
+constexpr int RES_WARPS = 4;
+__global__ void __launch_bounds__(32 * RES_WARPS) k_results(const uint64_t *__restrict__ seeds, const SeedNoise *__restrict__ noise, const float *__restrict__ mx,
                           const uint32_t *__restrict__ nbuck, const uint32_t *__restrict__ nsites, const Site *__restrict__ sites,
                           Eval *__restrict__ ev, const uint32_t *__restrict__ nev, const int32_t *__restrict__ f4, const FloodStat *__restrict__ st4,
                           Params P, dsg_search_seed *__restrict__ out, dsg_search_row *__restrict__ rows, uint32_t *ctr) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t s = blockIdx.x * RES_WARPS + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
     if (s >= ctr[C_NS]) return;
     Eval *E = ev + size_t(s) * EVC;
     const uint32_t ne = nev[s];
-    double best = 0;
-    for (int k2 = 0; k2 < EXN && uint32_t(k2) < ne; k2++) {
-        Eval &e = E[k2];
-        const int32_t j = f4[s * EXN + k2];
-        if (j >= 0) { e.s4 = st4[j].cells * 16.0 * 16 / 1e6; e.edge |= st4[j].edge != 0; }
-        if (!e.exact || e.nostart) continue;
-        best = fmax(best, e.s4 > 0 ? e.s4 : e.s8);
-    }
+    double best = 0;                                     // lane 0's
+    if (lane == 0)
+        for (int k2 = 0; k2 < EXN && uint32_t(k2) < ne; k2++) {
+            Eval &e = E[k2];
+            const int32_t j = f4[s * EXN + k2];
+            if (j >= 0) { e.s4 = st4[j].cells * 16.0 * 16 / 1e6; e.edge |= st4[j].edge != 0; }
+            if (!e.exact || e.nostart) continue;
+            best = fmax(best, e.s4 > 0 ? e.s4 : e.s8);
+        }
+    __syncwarp();
+    const auto row_of = [&](uint32_t k) { return k < ne && !(E[k].proxy < P.csv_min && E[k].s8 <= 0 && E[k].s4 <= 0); };
     uint32_t nr = 0;
-    for (uint32_t k = 0; k < ne; k++) nr += !(E[k].proxy < P.csv_min && E[k].s8 <= 0 && E[k].s4 <= 0);
-    uint32_t at = nr ? atomicAdd(ctr + C_ROWS, nr) : 0;
-    if (at + nr > ROWCAP) { atomicOr(ctr + C_FLAGS, F_ROWS); nr = 0; }
-    dsg_search_seed &o = out[s];
-    o.seed = seeds[s];
-    o.fya = noise[s].oct[0].fy; o.fyb = noise[s].oct[2].fy;       // octave -10 of the temperature, sides A and B
-    o.maxta = mx[2 * s]; o.maxtb = mx[2 * s + 1];
-    o.candidates = nbuck[s]; o.sites = nsites[s]; o.best = best; o.row0 = at; o.nrows = nr;
+    for (uint32_t k0 = 0; k0 < ne; k0 += 32) nr += uint32_t(__popc(__ballot_sync(0xffffffffu, row_of(k0 + lane))));
+    uint32_t at = 0;
+    if (nr && lane == 0) at = atomicAdd(ctr + C_ROWS, nr);
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (at + nr > ROWCAP) { if (lane == 0) atomicOr(ctr + C_FLAGS, F_ROWS); nr = 0; }
+    if (lane == 0) {
+        dsg_search_seed &o = out[s];
+        o.seed = seeds[s];
+        o.fya = noise[s].oct[0].fy; o.fyb = noise[s].oct[2].fy;       // octave -10 of the temperature, sides A and B
+        o.maxta = mx[2 * s]; o.maxtb = mx[2 * s + 1];
+        o.candidates = nbuck[s]; o.sites = nsites[s]; o.best = best; o.row0 = at; o.nrows = nr;
+    }
     if (!nr) return;
-    for (uint32_t k = 0; k < ne; k++) {
-        const Eval &e = E[k];
-        if (e.proxy < P.csv_min && e.s8 <= 0 && e.s4 <= 0) continue;
-        const Site &st = sites[size_t(s) * MS + e.rank];
-        dsg_search_row &r = rows[at++];
-        r.seed = seeds[s]; r.rank = e.rank; r.x = e.x; r.z = e.z;
-        r.score = st.s; r.t0 = st.t; r.c0 = st.c; r.e0 = st.e;
-        r.proxy = e.proxy; r.s8 = e.s8; r.s4 = e.s4; r.hot = e.hot;
-        r.edge = e.edge; r.exact = e.exact && !e.nostart && k < uint32_t(P.exact_n) ? 1 : 0;
+    for (uint32_t k0 = 0; k0 < ne; k0 += 32) {
+        const uint32_t k = k0 + lane;
+        const bool on = row_of(k);
+        const uint32_t m = __ballot_sync(0xffffffffu, on);
+        if (on) {
+            const Eval e = E[k];
+            const Site &st = sites[size_t(s) * MS + e.rank];
+            dsg_search_row &r = rows[at + __popc(m & ((1u << lane) - 1))];
+            r.seed = seeds[s]; r.rank = e.rank; r.x = e.x; r.z = e.z;
+            r.score = st.s; r.t0 = st.t; r.c0 = st.c; r.e0 = st.e;
+            r.proxy = e.proxy; r.s8 = e.s8; r.s4 = e.s4; r.hot = e.hot;
+            r.edge = e.edge; r.exact = e.exact && !e.nostart && k < uint32_t(P.exact_n) ? 1 : 0;
+        }
+        at += uint32_t(__popc(m));
     }
 }
 // Tiles taken in this wave back to zero (the next wave allocates from tile 0 again).
@@ -1050,7 +1108,7 @@ void capture_wave(Pipeline &p, Slot &S) {
     capture_phase(p, S, 1);
     k_cover_pairs<<<8 * 148, 256, 0, S.st>>>(S.hot, S.nsites, S.f1, S.f2, FloodView{S.ph[0].ctl, S.ph[0].dir}, FloodView{S.ph[1].ctl, S.ph[1].dir},
                                               S.ph[0].st, S.pool.T, p.P, S.cvm, S.ctr);
-    k_cover<<<(SC + 7) / 8, 256, 0, S.st>>>(S.hot, S.nsites, S.f1, S.f2, S.ph[0].st, S.ph[1].st, p.P, S.cvm, S.nzone, S.zslot, S.zmslot, S.ctr);
+    k_cover<<<SC, COVER_THREADS, 0, S.st>>>(S.hot, S.nsites, S.f1, S.f2, S.ph[0].st, S.ph[1].st, p.P, S.cvm, S.nzone, S.zslot, S.zmslot, S.ctr);
     k_stamp<<<1, 1, 0, S.st>>>(ts, 5);
     k_zone_list<<<1, LIST_THREADS, 0, S.st>>>(S.nzone, S.zslot, S.zmslot, S.zfirst, S.zones, S.zmeta, S.chunks, S.ctr, p.c.zcap, p.c.cellcap, p.c.chcap);
     DSG_CU(cudaGetLastError());
@@ -1063,7 +1121,7 @@ void capture_wave(Pipeline &p, Slot &S) {
     k_comp_scatter<<<64, 256, 0, S.st>>>(S.rec, S.ctr, S.zoff, S.zfill, S.zcomp2);
     k_comp_order<<<4 * 148, 256, 0, S.st>>>(S.rec, S.ctr, S.zoff, S.zcomp2, S.zcomp);
     DSG_CU(cudaFuncSetAttribute(k_evals, cudaFuncAttributeMaxDynamicSharedMemorySize, int(EV_SMEM)));
-    k_evals<<<(SC + EV_WARPS - 1) / EV_WARPS, EV_WARPS * 32, EV_SMEM, S.st>>>(S.zfirst, S.zones, S.zmeta, S.zoff, S.zcomp, S.rec, p.P, S.evu,
+    k_evals<<<SC, EV_THREADS, EV_SMEM, S.st>>>(S.zfirst, S.zones, S.zmeta, S.zoff, S.zcomp, S.rec, p.P, S.evu,
                                                                              S.ekey, S.nev, S.ctr);
     DSG_CU(cudaFuncSetAttribute(k_eval_order, cudaFuncAttributeMaxDynamicSharedMemorySize, int(EVO_SMEM)));
     k_eval_order<<<SC, EVO_THREADS, EVO_SMEM, S.st>>>(S.evu, S.ekey, S.nev, p.P, S.ev, S.tries, S.ctr);
@@ -1077,7 +1135,7 @@ void capture_wave(Pipeline &p, Slot &S) {
     k_stamp<<<1, 1, 0, S.st>>>(ts, 7);
     k_retry<<<16, 256, 0, S.st>>>(S.tries, S.f8, S.ph[2].st, S.ph[2].ctl, S.ev, S.nev, p.P, S.ctr, S.ph[3].ctl, S.f4);
     capture_phase(p, S, 3);
-    k_results<<<(SC + 127) / 128, 128, 0, S.st>>>(S.seeds, S.noise, S.mx, S.nbuck, S.nsites, S.sites, S.ev, S.nev, S.f4, S.ph[3].st, p.P, S.out,
+    k_results<<<(SC + RES_WARPS - 1) / RES_WARPS, 32 * RES_WARPS, 0, S.st>>>(S.seeds, S.noise, S.mx, S.nbuck, S.nsites, S.sites, S.ev, S.nev, S.f4, S.ph[3].st, p.P, S.out,
                                                    S.rows, S.ctr);
     k_pool_zero<<<8 * 148, 256, 0, S.st>>>(S.pool.T, S.ctr, S.pool.cap);
     k_wave_end<<<1, 1, 0, S.st>>>(S.ctr);
