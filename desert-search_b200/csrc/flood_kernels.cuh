@@ -164,6 +164,7 @@ static __global__ void __launch_bounds__(EVAL_THREADS, DSG_EVAL_MINB) k_tile_eva
         PendingState pend[EVAL_THREADS];
         struct { ExactTab exact; PendingState pend[EVAL_THREADS / 4]; } split;
     } s_u;
+    __shared__ ShiftLines s_shift;
     __shared__ int8_t s_res[EVAL_THREADS];
     __shared__ int s_n;
     __shared__ uint32_t s_run;
@@ -248,9 +249,10 @@ static __global__ void __launch_bounds__(EVAL_THREADS, DSG_EVAL_MINB) k_tile_eva
                 const int bi = int(pos & 0xffff) * TILE + int(sb & 3) * SUB, bj = int(pos >> 16) * TILE + int(sb >> 2) * SUB;
                 patch_build(s_noise, s_u.patch, double(c.qx + (bi - c.half) * c.step) - 2, double(c.qz + (bj - c.half) * c.step) - 2,
                             double((SUB - 1) * c.step + 4), int(threadIdx.x), EVAL_THREADS);
+                shift_build(s_noise, s_shift, c.qx + (bi - c.half) * c.step, c.qz + (bj - c.half) * c.step, c.step, int(threadIdx.x));
                 __syncthreads();
                 PendingState p;
-                if (on) v = desert_state_begin_patch(s_noise, s_u.patch, w, x, z, p);
+                if (on) v = desert_state_begin_patch(s_noise, s_u.patch, s_shift, w, x, z, int(threadIdx.x & 15), int(threadIdx.x >> 4), p);
                 __syncthreads();                          // the pending points take the patch's place
                 int slot = -1;
                 if (v < 0) { slot = atomicAdd(&s_n, 1); s_u.pend[slot] = p; }
