@@ -285,7 +285,7 @@ static __global__ void __launch_bounds__(EVAL_THREADS, DSG_EVAL_MINB) k_tile_eva
 // cells lie on a grid, so an octave's position, fraction, fade and column hashes depend on the column alone and its
 // fraction, fade and lattice row on the row alone: 128 threads work them out once per sub-block.  A corner then is one
 // hash lookup, its gradient (gx and gz packed in a word, gy * dy from a table per octave: the reference's u + v as in
-// LatticePoint) and two multiply-adds.  Measured on 222 gated seeds (51,146 step-256 floods, 200,683 sub-blocks; then 4,505
+// LatticePoint) and two multiply-adds.  Bound by shared-memory wavefronts (77%), then issue (73%).  Measured on 222 gated seeds (51,146 step-256 floods, 200,683 sub-blocks; then 4,505
 // step-128 floods): the pre-flood stage 3.23 -> 2.69 ms, the step-128 stage 1.53 -> 1.37 ms against k_tile_eval.
 struct __align__(16) HotNoise {
     NOct oct[4];                                          // T: side A's two octaves, then side B's
