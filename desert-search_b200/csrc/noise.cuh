@@ -147,7 +147,11 @@ __device__ __forceinline__ int patch_slot(int i) {          // -1: not kept
 }
 __device__ __forceinline__ int patch_octave(int slot) { return slot + (slot < 14 ? 0 : slot < 20 ? 3 : slot < 28 ? 6 : 12); }
 // The table of the patch [x0, x0 + ext] x [z0, z0 + ext] (quarts, the warped coordinates included) by `nt` threads.  An
-// octave whose patch spans more than about a lattice cell is left out (bx infinite: no cell is found inside).
+// octave whose patch spans more than about a lattice cell is left out (bx infinite: no cell is found inside).  So is one whose
+// corner lies in lattice cell -1 or -2 along either axis.  A point of such a patch may lie in (-1, 1) and its difference from
+// the corner in [1, 2), where doubles are coarser than the point's own: the last bits of its fraction would be lost.
+// Everywhere else the difference is exact: from 0 it is the point itself, from any other corner the point is at least 1 in
+// magnitude, so both are multiples of 2^-52.  The two cells are next to the origin of the octave's own noise.
 __device__ __forceinline__ void patch_build(const SeedNoise &S, PatchCache &C, double x0, double z0, double ext, int t, int nt) {
     for (int k = t; k < kPatchOct * 9; k += nt) {
         const int slot = k / 9, j = k % 9, i = patch_octave(slot);
@@ -155,7 +159,7 @@ __device__ __forceinline__ void patch_build(const SeedNoise &S, PatchCache &C, d
         const uint8_t *P = S.perm[i];
         const double s = (kSideB >> i & 1) ? 337. / 331. : 1.;
         const double bx = floor(x0 * s * o.freq + o.ox), bz = floor(z0 * s * o.freq + o.oz);
-        const bool use = ext * s * o.freq < 1.25;
+        const bool use = ext * s * o.freq < 1.25 && (bx < -2 || bx >= 0) && (bz < -2 || bz >= 0);
         if (j == 0) { C.bx[slot] = use ? bx : __longlong_as_double(0x7ff0000000000000ll); C.bz[slot] = bz; }
         if (!use) continue;
         const int ix = (int(bx) + j % 3) & 255, iz = (int(bz) + j / 3) & 255, a = P[ix] + o.iy;
@@ -172,7 +176,7 @@ __device__ __forceinline__ double perlin_patch(const NOct &o, const uint8_t *__r
     // both in [0, 2): compared as integers (a negative number's sign bit is the largest)
     if (k < 0 || uint32_t(__double2hiint(fx)) >= 0x40000000u || uint32_t(__double2hiint(fz)) >= 0x40000000u) return perlin(o, P, G, x, 0, z);
     const bool cx = __double2hiint(fx) >= 0x3ff00000, cz = __double2hiint(fz) >= 0x3ff00000;
-    fx -= cx ? 1. : 0.; fz -= cz ? 1. : 0.;        // the fractions x - floor(x), z - floor(z): every step is exact
+    fx -= cx ? 1. : 0.; fz -= cz ? 1. : 0.;        // the fractions x - floor(x), z - floor(z): exact for the corners patch_build keeps
     const LatticePoint *q = &C.pt[k][(cz ? 3 : 0) + (cx ? 1 : 0)];
     const double tx = fade_d(fx), tz = fade_d(fz), ty = o.vy, ex = fx - 1;
     const auto row = [&](const LatticePoint &a, const LatticePoint &b, double dz) {
