@@ -52,7 +52,7 @@ template <class F> __device__ __forceinline__ void each_chunk(const DZone *__res
 // FP64 chains (FP64 pipe 50%, issue 50%, shared-memory wavefronts 61%, 4 blocks of 8 warps per SM by registers).  A cell
 // per thread, every corner loaded, was bound by shared memory (78% of its wavefronts; 350 us); rows that test one by one
 // for a new lattice row serialised (316 us); 2 or 3 blocks per SM without spills 314 and 277 us.
-// A zone narrower than 8 cells is evaluated cell by cell: most of a tile would lie outside it.
+// A zone narrower than 8 cells, or one whose coordinates wrap, is evaluated cell by cell (zones::tiled).
 constexpr int PT = 32, POCT = 14;                         // tile side; octaves: T (A 0-1, B 0-1), C 0-2 (A, B), E 0-1 (A, B)
 struct ProxyOct { int oct, side, log2f; };                // octave in SeedNoise, side, -log2 of its frequency
 constexpr ProxyOct kPO[POCT] = {{0, 0, 10}, {1, 0, 8}, {2, 1, 10}, {3, 1, 8}, {8, 0, 9}, {9, 0, 8}, {10, 0, 7}, {17, 1, 9}, {18, 1, 8}, {19, 1, 7},
@@ -147,9 +147,9 @@ __global__ void __launch_bounds__(256, DSG_PROXY_MINB) k_proxy(const SeedNoise *
     int staged = -1;
     each_chunk(zones, wk, [&](uint32_t, const DZone &z, int64_t c0, int64_t c1) {
         const SeedNoise &S = noise[z.seed];
-        if (z.nx < 8 || z.nz < 8) {                       // a strip: most of a tile would lie outside
+        if (!zones::tiled(z)) {                           // cell by cell, coordinates modulo 2^32
             for (int64_t c = c0 + threadIdx.x; c < c1; c += blockDim.x)
-                out[z.off + c] = proxy_prob(S, w, z.x0 + 32 * int(c % z.nx), z.z0 + 32 * int(c / z.nx)) >= cut;
+                out[z.off + c] = proxy_prob(S, w, int(uint32_t(z.x0) + 32u * uint32_t(c % z.nx)), int(uint32_t(z.z0) + 32u * uint32_t(c / z.nx))) >= cut;
             return;
         }
         if (z.seed != staged) {                           // block-uniform: every thread walks the same chunks
