@@ -47,7 +47,13 @@ namespace gate {
 struct __align__(16) Oct { uint8_t perm[256]; double ox, oz, fy, vy; int32_t iy, pad[3]; };
 static_assert(sizeof(Oct) == 304, "Oct layout");
 
-constexpr float AMP_E2 = 3e-5f;                    // 2 E
+// 2 E.  A wider window lists more cells and drops fewer seeds, and the amplitudes are the same: the tests build it wider
+// to fill the lists, which ordinary seeds do not.
+#ifndef DSG_AMP_WINDOW
+#define DSG_AMP_WINDOW 3e-5f
+#endif
+constexpr float AMP_E2 = DSG_AMP_WINDOW;
+static_assert(AMP_E2 >= 3e-5f, "the error bound");
 constexpr float AMP_FLOOR = 0.24f;                 // amplitudes below it are rare: no cell under it is listed at first
 constexpr int AMP_CAP = 32;                        // listed cells per warp
 
@@ -96,6 +102,7 @@ __device__ __forceinline__ float warp_max(float v) {
 
 // ---------------------------------------------------------------- listed cells of a warp
 struct CellList { uint32_t pos[AMP_CAP]; float val[AMP_CAP]; };
+static_assert(AMP_CAP == 32, "list_cells clears a full list with a lane per entry");
 // Running state of a warp's pass over its cells (warp-uniform): the maximum of the cells listed so far, the value
 // from which cells are listed, the number listed.
 struct Run { float best, lim; int n; };
