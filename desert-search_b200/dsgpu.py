@@ -237,7 +237,9 @@ class Component(C.Structure):
                 ("inner", C.c_uint32), ("pick", C.c_int32 * 3)]
 
 
+# the same record as an array element
 COMPONENT = np.dtype([("zone", "<u4"), ("first", "<i4"), ("cells", "<u4"), ("minx", "<i4"), ("minz", "<i4"), ("inner", "<u4"), ("pick", "<i4", (3,))])
+assert COMPONENT.itemsize == C.sizeof(Component)
 
 
 def proxy_components(seeds, zone_seed, zones, min_cells=1, cap=1 << 16):
