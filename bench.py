@@ -24,7 +24,7 @@ stage boundaries of the wave graph).  Besides it, the default run adds (single G
 device pipeline, per-stage path on one host worker (the plain form: one batched call per stage with host syncs
 between stages), per-stage path on 8 workers, and the reference's own GPU searcher; wall clock; outputs
 compared), "default_mode" (the reference's default command line, ours vs its CPU searcher), "gate" (the seed
-gate alone against the shared-memory roofline, and the reference's tgate on the same seeds) and "flood" (exact
+gate alone against its issue and shared-memory rooflines, and the reference's tgate on the same seeds) and "flood" (exact
 step-1 floods of uneven size: one batch, the flood service under Poisson arrivals, sequential per-request
 launches under the same arrivals, the reference's dflood on the host cores, FP64 roofline).
 """
@@ -48,17 +48,23 @@ UNIT = "gated seeds/s"
 START = 2 * 10**13
 PER_STEP = 1 << 24
 RANK_STRIDE = 10**12            # per-GPU seed ranges, as deploy/prun.sh assigns them
-# pre-gate screen: 2 sides x 256 rows x 267 lattice columns x 16 bytes of sequence values (two hashes) per phase-passed seed
+# k_amp256 (the pre-gate): warp instructions per phase-passed seed, from one ncu capture (smsp__inst_executed.sum 657,989,826 over
+# 7,618 seeds on 2^20 seed indices)
+PRE_INST_PER_SEED = 657_989_826 / 7618
+INST_PER_CLK_PER_SM = 4         # one per scheduler
+# its screen: 2 sides x 256 rows x 267 lattice columns x 16 bytes of sequence values (two hashes) per phase-passed seed
 PRE_BYTES_PER_SEED = 2 * 256 * 267 * 16
 SMEM_BYTES_PER_CLK_PER_SM = 128  # 32 banks x 4 bytes
 FP64_FLOPS_PER_CLK_PER_SM = 128  # 64 FP64 FMA lanes per SM (B200) x 2 flops
 # k_amp256 DRAM traffic per phase-passed seed from one ncu capture (dram__bytes_read.sum + write.sum =
 # 37.0 MB + 0.1 MB over 60,230 seeds on 2^23 seed indices): the seed's octave table read once
 PRE_DRAM_BYTES_PER_SEED = (37.0e6 + 0.1e6) / 60230
-# k_tile_eval FP64 work per evaluated cell: executed DADD + DMUL + 2 x DFMA (ncu counters over every k_tile_eval
-# launch) divided by the cells of the evaluated 16x16 sub-blocks, on exact step-1 floods of the 32 largest verified
-# finds (2,297 on step-8 floods of the 6 largest).  Counted with each gradient as one DADD, the reference's
-# arithmetic; the kernel now forms it as a DMUL and two DFMAs, which this count does not credit.
+# FP64 work per evaluated cell of an exact flood in the reference's arithmetic: DADD + DMUL + 2 x DFMA that an earlier
+# k_tile_eval executed (ncu counters over every launch) divided by the cells of the evaluated 16x16 sub-blocks, on exact
+# step-1 floods of the 32 largest verified finds (2,297 on step-8 floods of the 6 largest).  That kernel did the reference's
+# operations one for one, cell by cell, each gradient one DADD.  The present kernel shares a sub-block's lattice points and
+# forms gradients with fused multiply-adds: 1,257 DADD, 1,072 DMUL and 788 DFMA per evaluated cell on step-1 floods of 24
+# finds, 3,904 flops.  So this count is a measure of work done for the caller, below what the kernel executes.
 EVAL_FP64_FLOPS_PER_CELL = 2829
 
 
@@ -192,19 +198,23 @@ def search_steps(dsgpu, base, steps, warmup, per_step):
 # ---------------------------------------------------------------------------- the gate alone
 def gate_leg(dsgpu, sm_mhz, sms, steps=6, warmup=3):
     """The seed gate (y-phase, octave init, pre-gate, full gate) alone on 2^26 indices per step, its pre-gate
-    kernel (k_amp256) against the shared-memory roofline, and the reference's tgate (its GPU gate) on the same seeds."""
+    kernel (k_amp256) against its issue and shared-memory rooflines, and the reference's tgate (its GPU gate) on the same seeds."""
     n = 1 << 26
     ms, mk, counts = dsgpu.gate_bench(START, n, steps, warmup)
     pre_ms = float(mk[2])
-    achieved = counts[1] * PRE_BYTES_PER_SEED / (pre_ms / 1e3) / 1e9
-    peak = sms * SMEM_BYTES_PER_CLK_PER_SM * sm_mhz * 1e6 / 1e9
+    achieved = counts[1] * PRE_INST_PER_SEED / (pre_ms / 1e3) / 1e9
+    peak = sms * INST_PER_CLK_PER_SM * sm_mhz * 1e6 / 1e9
+    smem = counts[1] * PRE_BYTES_PER_SEED / (pre_ms / 1e3) / 1e9
+    smem_peak = sms * SMEM_BYTES_PER_CLK_PER_SM * sm_mhz * 1e6 / 1e9
     out = {"seeds_per_step": n, "steps": steps, "gated_per_s": counts[3] / (ms / 1e3), "seeds_per_s": counts[0] / (ms / 1e3),
            "kernel_ms": {"phase": float(mk[0]), "octave_init": float(mk[1]), "pregate": pre_ms, "fullgate": float(mk[3])},
            "counts": {"seeds": int(counts[0]), "phase_passed": int(counts[1]), "pre_passed": int(counts[2]), "gated": int(counts[3])},
-           "roofline": {"bound": "smem", "kernel": "k_amp256", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+           "roofline": {"bound": "issue", "kernel": "k_amp256", "achieved": achieved, "peak": peak, "unit": "Ginst/s", "frac": achieved / peak,
+                        "smem": {"achieved": smem, "peak": smem_peak, "unit": "GB/s", "frac": smem / smem_peak},
                         "traffic": counts[1] / steps * PRE_DRAM_BYTES_PER_SEED,
-                        "note": "shared-memory bytes of the screen (16 per cell and lattice column) / k_amp256 event time; peak = SMs x 128 B/clk "
-                                "at the median sampled SM clock; traffic = DRAM bytes per launch scaled from an ncu capture"}}
+                        "note": "warp instructions (ncu count per phase-passed seed) / k_amp256 event time; peak = SMs x 4 per clk at the median "
+                                "sampled SM clock; smem: the screen's bytes (16 per cell and lattice column), peak = SMs x 128 B/clk; "
+                                "traffic = DRAM bytes per launch scaled from an ncu capture"}}
     tg = ref_exe("tgate")
     if tg:
         t0 = time.perf_counter()
@@ -412,7 +422,7 @@ def bench_floods(dsgpu, sm_mhz, sms, n_small=4096, n_large=4096, rates=(100.0, 5
     if EVAL_FP64_FLOPS_PER_CELL:
         ach = EVAL_FP64_FLOPS_PER_CELL * evaluated / t_batch
         batch["roofline"] = {"bound": "fp64", "kernel": "k_tile_eval", "achieved": ach / 1e12, "peak": peak / 1e12, "unit": "TFLOP/s",
-                             "frac": ach / peak, "note": "FP64 flops per evaluated cell in the reference arithmetic (ncu count, one add per gradient) x cells evaluated / batch wall time; "
+                             "frac": ach / peak, "note": "FP64 flops per evaluated cell in the reference's arithmetic (the kernel executes more: 3,904 against 2,829) x cells evaluated / batch wall time; "
                                                          "peak = SMs x 64 FP64 FMA/clk x 2 at the sampled clock (nominal rate)"}
     out = {"batch": batch}
     # the reference's dflood on the host cores: a sample of small sites and large sites

@@ -28,7 +28,8 @@
 //
 // What bounds them, on a B200 at 1,965 MHz, 2^26 seed indices (482,670 phase-passed seeds, 31,114 full-gate seeds):
 // register operands and instruction issue.  Per cell and lane the 256^2 screen issues 20.9 instructions (13.5 of them
-// on the FMA pipe) and reads 16 bytes of shared memory: issue 70% active, FMA pipe 60%, shared-memory wavefronts 59%.
+// on the FMA pipe) and reads 16 bytes of shared memory: issue 69% of active cycles, the FMA pipe busy in 62% (a two-wide
+// instruction holds it for two; by instructions 50%), shared-memory wavefronts 59%.
 // Before, every cell gathered its 18 (or 8) corner terms: the pre-gate took 161 ms (now 52), the full gate 43.6 (now
 // 15.4), the sub-grid form 21.7 ms for 84,414 seeds (now 8.3).  Measured on the way: a multiply-add of three distinct
 // registers takes 1.56 cycles per scheduler, of two and a constant 1.16, the two-wide one 3 (so two-wide forms serve

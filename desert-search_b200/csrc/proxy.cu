@@ -49,7 +49,7 @@ template <class F> __device__ __forceinline__ void each_chunk(const DZone *__res
 // where it took 69 and 137 others.  The values are the same doubles: the same expressions, evaluated once per column or row.
 // C and E follow only where a cell of the tile is hot.
 // Measured (B200, 160 zones of about 195 x 195 cells): 412 us before, 266 now; one launch is bound by the latency of its
-// FP64 chains (FP64 pipe 50%, issue 50%, shared-memory wavefronts 61%, 4 blocks of 8 warps per SM by registers).  A cell
+// FP64 chains (FP64 pipe 52%, issue 52%, shared-memory wavefronts 68%, 4 blocks of 8 warps per SM by registers).  A cell
 // per thread, every corner loaded, was bound by shared memory (78% of its wavefronts; 350 us); rows that test one by one
 // for a new lattice row serialised (316 us); 2 or 3 blocks per SM without spills 314 and 277 us.
 // A zone narrower than 8 cells, or one whose coordinates wrap, is evaluated cell by cell (zones::tiled).
